@@ -11,13 +11,15 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libpgm_b200.so"
-SOURCES = [CSRC / "engine.cu", CSRC / "capi.cpp"]
+SOURCES = [CSRC / "engine.cu", CSRC / "transforms.cu", CSRC / "capi.cpp"]
 HEADERS = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [ROOT / "include" / "pgm_b200.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -44,14 +46,21 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if not force and not needs_build():
         return LIB
     tmp = LIB.with_suffix(".so.tmp")
-    cmd = [nvcc(), *ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-shared",
-           "-o", str(tmp), *map(str, SOURCES), "-lcufft", f"-L{cuda_lib_dir()}",
-           f"-Xlinker", f"-rpath,{cuda_lib_dir()}"]
-    if verbose:
-        print(" ".join(cmd))
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + r.stdout + r.stderr)
+
+    def run(cmd):
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError("nvcc failed:\n" + r.stdout + r.stderr)
+
+    with tempfile.TemporaryDirectory() as d:   # the sources side by side, then the link
+        objects = [str(Path(d) / (p.stem + ".o")) for p in SOURCES]
+        flags = [*ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-O2"]
+        with ThreadPoolExecutor() as pool:
+            list(pool.map(run, [[nvcc(), *flags, "-c", "-o", o, str(p)] for p, o in zip(SOURCES, objects)]))
+        run([nvcc(), *ARCH, "-shared", "-o", str(tmp), *objects, "-lcufft", f"-L{cuda_lib_dir()}",
+             "-Xlinker", f"-rpath,{cuda_lib_dir()}"])
     tmp.replace(LIB)
     return LIB
 

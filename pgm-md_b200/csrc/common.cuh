@@ -457,4 +457,37 @@ __device__ __forceinline__ bool chunkFinish(const Dev& dv, int chunk, int s, dou
     return true;
 }
 
+// A grid index within one period of [0, K), wrapped.
+__device__ __forceinline__ int wrapIndex(int g, int K) {
+    g += (g < 0) ? K : 0;
+    g -= (g >= K) ? K : 0;
+    return g;
+}
+
+// The mixed spread's 64-bit fixed point: contributions rounded to multiples of 2^-32 and added as integers, so
+// the grid's sums do not depend on the order of the atomics (the evaluation repeats bit for bit); the grid is
+// converted to float once before the transforms.
+constexpr float GRID_FIX_SCALE = 4294967296.0f;   // 2^32
+__device__ __forceinline__ void gridFixAdd(long long* g, float v) {
+    atomicAdd((unsigned long long*) g, (unsigned long long) __float2ll_rn(v * GRID_FIX_SCALE));
+}
+__device__ __forceinline__ float gridFixTake(long long* g) {   // the value, and the word cleared for the next spread
+    const long long v = *g;
+    *g = 0;
+    return (float) ((double) v * (1.0 / 4294967296.0));
+}
+
+// The initial guess x0 of component g = 3 gi + k when it does not depend on b (guess 1: zero; 2: history slot;
+// 3: mu3 from history; 4: mu4 from history) (core/pgm_core.cpp:309-329).
+__device__ __forceinline__ double historyGuess(const Dev& dv, int guess, size_t g, size_t hs) {
+    const int h0 = dv.ctl->h[0], h1 = dv.ctl->h[1], h2 = dv.ctl->h[2], h3 = dv.ctl->h[3];
+    switch (guess) {
+    case 1: return 0.0;
+    case 2: return dv.hist[h0 * hs + g];
+    case 3: return 3 * dv.hist[h0 * hs + g] - 3 * dv.hist[h1 * hs + g] + dv.hist[h2 * hs + g];
+    default:
+        return 4 * dv.hist[h0 * hs + g] - 6 * dv.hist[h1 * hs + g] + 4 * dv.hist[h2 * hs + g] - dv.hist[h3 * hs + g];
+    }
+}
+
 }  // namespace pgmb200

@@ -10,6 +10,7 @@
 #include "lines.cuh"
 #include "tiles.cuh"
 #include "pgm_engine.h"
+#include "transforms.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -1168,26 +1169,6 @@ struct Engine::Impl {
         return clusters > 0;
     }
 
-    // The grid-transform kernel: compiled for one cubic grid size (32, 40, 48, 64), or for any grid; energy: the
-    // final pass's variant that also sums the reciprocal energy and strain.
-    template <typename R> static void (*fftgKernel(int kc, bool energy = false))(Dev, int) {
-        if (energy)
-            switch (kc) {
-            case 32: return k_fft_grid<R, 32, true>;
-            case 40: return k_fft_grid<R, 40, true>;
-            case 48: return k_fft_grid<R, 48, true>;
-            case 64: return k_fft_grid<R, 64, true>;
-            default: return k_fft_grid<R, 0, true>;
-            }
-        switch (kc) {
-        case 32: return k_fft_grid<R, 32>;
-        case 40: return k_fft_grid<R, 40>;
-        case 48: return k_fft_grid<R, 48>;
-        case 64: return k_fft_grid<R, 64>;
-        default: return k_fft_grid<R, 0>;
-        }
-    }
-
     // Attributes of the grid-transform kernel; false when its blocks (a block per x-plane of every system) cannot
     // all be resident at once on this GPU or a block's shared memory does not fit.
     template <typename R> bool prepareGrid() {
@@ -1197,16 +1178,16 @@ struct Engine::Impl {
         CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, devId));
         if (!coop || fftgSmem > (size_t) optin)
             return false;
-        CU(cudaFuncSetAttribute((const void*) fftgKernel<R>(fftgKc), cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CU(cudaFuncSetAttribute((const void*) gridKernel<R>(fftgKc, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int) fftgSmem));
         int perSm = 0;
-        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fftgKernel<R>(fftgKc), FftgThreads<R>::n,
+        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, gridKernel<R>(fftgKc, false), FftgThreads<R>::n,
                                                          fftgSmem));
         // the final pass's variant: every block resident too, and a conv partial of its own for each x-plane
-        CU(cudaFuncSetAttribute((const void*) fftgKernel<R>(fftgKc, true),
+        CU(cudaFuncSetAttribute((const void*) gridKernel<R>(fftgKc, true),
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fftgSmem));
         int perSmE = 0;
-        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSmE, fftgKernel<R>(fftgKc, true), FftgThreads<R>::n,
+        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSmE, gridKernel<R>(fftgKc, true), FftgThreads<R>::n,
                                                          fftgSmem));
         gridEnergyOk = (long long) perSmE * sms >= (long long) maxK0 * nsys && maxK0 <= convBlocks;
         return (long long) perSm * sms >= (long long) maxK0 * nsys;
@@ -1380,25 +1361,7 @@ struct Engine::Impl {
         CU(cudaGetLastError());
     }
 
-    // The persistent kernel for the pair lanes (8, 16 or 32; 4 runs as 8) and the grid's compile-time size.
-    // pass 0: the CG loop; 1 / 2: one field pass of dipoles (and charges).
-    typedef void (*PcgKernel)(Dev, int, const double*);
-    PcgKernel persistentKernel(int lanes, int pass = 0) {
-        const int kc = fftgKc;
-        auto pick = [&](auto gsTag) -> PcgKernel {
-            constexpr int GS = decltype(gsTag)::value;
-            if (kc == 48)
-                return pass == 0 ? k_cg_persistent<6, GS, 48, 0> : pass == 1 ? k_cg_persistent<6, GS, 48, 1>
-                                                                             : k_cg_persistent<6, GS, 48, 2>;
-            return pass == 0 ? k_cg_persistent<6, GS, 0, 0> : pass == 1 ? k_cg_persistent<6, GS, 0, 1>
-                                                                        : k_cg_persistent<6, GS, 0, 2>;
-        };
-        if (lanes >= 32)
-            return pick(std::integral_constant<int, 32>());
-        if (lanes >= 16)
-            return pick(std::integral_constant<int, 16>());
-        return pick(std::integral_constant<int, 8>());
-    }
+    PcgKernel persistentKernel(int lanes, int pass = 0) { return pcgKernel(lanes, fftgKc, pass); }
 
     // The whole CG loop (pass 0), or one field pass of the dipoles vec (1) and the charges (2): one cooperative
     // launch of the persistent kernel (one block per SM).
@@ -1485,7 +1448,7 @@ struct Engine::Impl {
         cfg.stream = sm;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        CU(cudaLaunchKernelEx(&cfg, fftgKernel<R>(fftgKc, energy), d, flags));
+        CU(cudaLaunchKernelEx(&cfg, gridKernel<R>(fftgKc, energy), d, flags));
     }
 
     // fix: the spread before went to the fixed-point grid (the grid kernel converts on its load, the others after a

@@ -6,30 +6,12 @@
 #pragma once
 
 #include "common.cuh"
+#include "gridfft.cuh"
 
 #include <cooperative_groups.h>
 #include <type_traits>
 
 namespace pgmb200 {
-
-__device__ __forceinline__ int wrapIndex(int g, int K) {
-    g += (g < 0) ? K : 0;
-    g -= (g >= K) ? K : 0;
-    return g;
-}
-
-// The mixed spread's 64-bit fixed point: contributions rounded to multiples of 2^-32 and added as integers, so
-// the grid's sums do not depend on the order of the atomics (the evaluation repeats bit for bit); the grid is
-// converted to float once before the transforms.
-constexpr float GRID_FIX_SCALE = 4294967296.0f;   // 2^32
-__device__ __forceinline__ void gridFixAdd(long long* g, float v) {
-    atomicAdd((unsigned long long*) g, (unsigned long long) __float2ll_rn(v * GRID_FIX_SCALE));
-}
-__device__ __forceinline__ float gridFixTake(long long* g) {   // the value, and the word cleared for the next spread
-    const long long v = *g;
-    *g = 0;
-    return (float) ((double) v * (1.0 / 4294967296.0));
-}
 
 // The fixed-point grid to the float grid (every point), clearing the fixed-point grid.
 __global__ void k_grid_from_fix(Dev dv) {
@@ -1066,7 +1048,6 @@ __global__ void __launch_bounds__(256) k_conv(Dev dv, int gateDone) {
 // Unnormalised, the spectrum in cuFFT's R2C / C2R layout F[(kx K1 + ky) (K2/2 + 1) + kz].  Each line transform is
 // a mixed-radix Stockham FFT (radices 4, 2, 3, 5; ping-pong buffers, no reordering pass) with twiddles
 // W^m = exp(-2 pi i m / K) from a table built on the host.
-constexpr int FFT_MAXK = 64;
 constexpr int FFTC_MAXC = 16;      // the largest cluster (a non-portable cluster size on sm_100)
 
 __host__ __device__ inline int fftRadices(int n, int* r) {
@@ -1077,66 +1058,6 @@ __host__ __device__ inline int fftRadices(int n, int* r) {
     while (n % 5 == 0) { r[c++] = 5; n /= 5; }
     return n == 1 ? c : -1;
 }
-
-// In-register DFT of length RAD, sign DIR (-1 forward, +1 inverse), unnormalised.
-template <typename R, int RAD, int DIR>
-__device__ __forceinline__ void smallDft(R* xr, R* xi) {
-    if (RAD == 2) {
-        const R ar = xr[0] + xr[1], ai = xi[0] + xi[1];
-        xr[1] = xr[0] - xr[1];
-        xi[1] = xi[0] - xi[1];
-        xr[0] = ar;
-        xi[0] = ai;
-    } else if (RAD == 3) {
-        const R s = (R) (DIR * 0.86602540378443864676);   // DIR sin(2 pi / 3)
-        const R tr = xr[1] + xr[2], ti = xi[1] + xi[2];
-        const R ur = xr[0] - (R) 0.5 * tr, ui = xi[0] - (R) 0.5 * ti;
-        const R dr = s * (xr[1] - xr[2]), di = s * (xi[1] - xi[2]);   // i s (v1 - v2) = (-di, dr)
-        xr[0] += tr;
-        xi[0] += ti;
-        xr[1] = ur - di;
-        xi[1] = ui + dr;
-        xr[2] = ur + di;
-        xi[2] = ui - dr;
-    } else if (RAD == 4) {
-        const R ar = xr[0] + xr[2], ai = xi[0] + xi[2], br = xr[0] - xr[2], bi = xi[0] - xi[2];
-        const R cr = xr[1] + xr[3], ci = xi[1] + xi[3];
-        const R er = xr[1] - xr[3], ei = xi[1] - xi[3];
-        const R dr = (R) (-DIR) * ei, di = (R) DIR * er;   // (v1 - v3) DIR i
-        xr[0] = ar + cr;
-        xi[0] = ai + ci;
-        xr[2] = ar - cr;
-        xi[2] = ai - ci;
-        xr[1] = br + dr;
-        xi[1] = bi + di;
-        xr[3] = br - dr;
-        xi[3] = bi - di;
-    } else {   // 5
-        const R c1 = (R) 0.30901699437494742410, c2 = (R) -0.80901699437494742410;   // cos(2 pi/5), cos(4 pi/5)
-        const R s1 = (R) (DIR * 0.95105651629515357212), s2 = (R) (DIR * 0.58778525229247312917);
-        const R a1r = xr[1] + xr[4], a1i = xi[1] + xi[4], a2r = xr[2] + xr[3], a2i = xi[2] + xi[3];
-        const R b1r = xr[1] - xr[4], b1i = xi[1] - xi[4], b2r = xr[2] - xr[3], b2i = xi[2] - xi[3];
-        const R p1r = xr[0] + c1 * a1r + c2 * a2r, p1i = xi[0] + c1 * a1i + c2 * a2i;
-        const R p2r = xr[0] + c2 * a1r + c1 * a2r, p2i = xi[0] + c2 * a1i + c1 * a2i;
-        const R q1r = s1 * b1r + s2 * b2r, q1i = s1 * b1i + s2 * b2i;   // y1 = p1 + i q1, y4 = p1 - i q1
-        const R q2r = s2 * b1r - s1 * b2r, q2i = s2 * b1i - s1 * b2i;   // y2 = p2 + i q2, y3 = p2 - i q2
-        xr[0] += a1r + a2r;
-        xi[0] += a1i + a2i;
-        xr[1] = p1r - q1i;
-        xi[1] = p1i + q1r;
-        xr[4] = p1r + q1i;
-        xi[4] = p1i - q1r;
-        xr[2] = p2r - q2i;
-        xi[2] = p2i + q2r;
-        xr[3] = p2r + q2i;
-        xi[3] = p2i - q2r;
-    }
-}
-
-// e / K for 0 <= e < 2^20, K >= 1 without an integer division: (e + 1/2) / K lies at least 1/(2K) from an
-// integer and the float product errs by at most about 2^-23 (e + 1/2) / K < 1/(8K), so truncation gives the
-// exact quotient.
-__device__ __forceinline__ int fdiv(int e, float invK) { return __float2int_rz(((float) e + 0.5f) * invK); }
 
 // Butterfly j of a Stockham pass of radix RAD (src = in + line start + j, dst = out + line start + (j / Ns) Ns RAD
 // + j mod Ns): reads src[r nb], twiddles by W^(r tws) (tws = (j mod Ns) N / (Ns RAD)), writes dst[r Ns].
@@ -1158,7 +1079,7 @@ __device__ __forceinline__ void stockhamButterfly(const typename CplxT<R>::T* sr
         xr[r] = v[r].x * w.x - v[r].y * wy;
         xi[r] = v[r].x * wy + v[r].y * w.x;
     }
-    smallDft<R, RAD, DIR>(xr, xi);
+    Dft<R, RAD, DIR>::run(xr, xi);
 #pragma unroll
     for (int r = 0; r < RAD; r++) {
         C o;
@@ -1216,40 +1137,6 @@ __device__ typename CplxT<R>::T* fftLines(typename CplxT<R>::T* a, typename Cplx
         b = t;
     }
     return a;
-}
-
-// The same passes for a compile-time length N: the radix sequence, strides and twiddle steps are constants and
-// the index divisions become multiplications.  NREM: the length still to transform, NS the earlier radices.
-template <typename R, int DIR, int N, int NREM, int NS>
-struct FftPassesC {
-    typedef typename CplxT<R>::T C;
-    static __device__ __forceinline__ C* run(C* a, C* b, int nlines, int ls, const C* tw) {
-        constexpr int RAD = NREM % 4 == 0 ? 4 : NREM % 2 == 0 ? 2 : NREM % 3 == 0 ? 3 : 5;
-        constexpr int nb = N / RAD, step = NREM / RAD;
-        for (int t = threadIdx.x; t < nlines * nb; t += blockDim.x) {
-            const int line = t / nb, j = t - line * nb;
-            const int q = j / NS, jn = j - q * NS;
-            stockhamButterfly<R, RAD, DIR>(a + line * ls + j, b + line * ls + q * NS * RAD + jn, nb, NS, jn * step,
-                                           tw);
-        }
-        __syncthreads();
-        return FftPassesC<R, DIR, N, NREM / RAD, NS * RAD>::run(b, a, nlines, ls, tw);
-    }
-};
-template <typename R, int DIR, int N, int NS>
-struct FftPassesC<R, DIR, N, 1, NS> {
-    typedef typename CplxT<R>::T C;
-    static __device__ __forceinline__ C* run(C* a, C*, int, int, const C*) { return a; }
-};
-
-// Line transforms of length N (the compile-time passes when KC > 0, which then equals N).
-template <typename R, int DIR, int KC>
-__device__ __forceinline__ typename CplxT<R>::T* fftLinesK(typename CplxT<R>::T* a, typename CplxT<R>::T* b,
-                                                           int nlines, int N, int ls, const typename CplxT<R>::T* tw) {
-    if constexpr (KC > 0)
-        return FftPassesC<R, DIR, KC, KC, 1>::run(a, b, nlines, ls, tw);
-    else
-        return fftLines<R, DIR>(a, b, nlines, N, ls, tw);
 }
 
 // Complex elements of each of the three transform buffers of a block of a cluster of C blocks for grid K (max
@@ -1451,259 +1338,11 @@ __global__ void __launch_bounds__(XL_THREADS) k_xlines(Dev dv, int gateDone) {
     }
 }
 
-// ------------------------------------------------------------------------------------------------ grid transforms
-
-// The transform pair with the influence product of a field pass as ONE cooperative kernel: block x of system s
-// (blockIdx.y; K0 blocks per system) owns x-plane x and, between two barriers of the system's blocks, a run of
-// the x-lines:
-//   1. plane x: its real rows two at a time as one complex row (x + i y), forward along z (real to half
-//      spectrum, separated by Hermitian symmetry) and along y in shared memory, stored to the spectrum
-//      F[(x K1 + ky) (K2/2 + 1) + kz];
-//   2. (barrier) lines l = ky (K2/2 + 1) + kz in [x lpb, x lpb + lpb): forward along x, the influence product,
-//      back along x, in place in the spectrum;
-//   3. (barrier) plane x back along y and z (imaginary parts at kz = 0 and the Nyquist index dropped, as a C2R
-//      transform does) into the real grid.
-// The same Stockham line transforms as the cluster kernel, with the exchange through L2 instead of distributed
-// shared memory, so a 48^3 grid spreads over 48 SMs.  Loads of what other blocks wrote bypass L1 (__ldcg).
-// Each barrier waits at most FFTG_SPIN_LIMIT polls; a block that gives up sets flags[11] and returns, and the
-// host reports the evaluation as failed.
-// Threads per block: 512 in float (64 registers, 2 blocks per SM), 256 in double (84 registers, 3 per SM).
-template <typename R> struct FftgThreads { static constexpr int n = 256; };
-template <> struct FftgThreads<float> { static constexpr int n = 512; };
-constexpr unsigned FFTG_SPIN_LIMIT = 1u << 22;   // polls of an L2 word (a few hundred ns each): about 1 s
-
-// Complex elements of each of the two transform buffers of a block for grid K (max of its plane rows, its
-// y-lines and its x-lines).
-__host__ __device__ inline int fftgBufferElems(const int* K) {
-    const int K2h = K[2] / 2 + 1, P = (K[1] + 1) / 2, ly = K[1] + 1, lx = K[0] + 1;
-    const int lpb = (K[1] * K2h + K[0] - 1) / K[0];
-    int m = P * K[2];
-    m = m > K2h * ly ? m : K2h * ly;
-    m = m > lpb * lx ? m : lpb * lx;
-    return (m + 1) / 2 * 2;   // 16-byte multiples
-}
-
-__device__ __forceinline__ unsigned ldAcquireGpu(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Barrier of nb blocks over an arrival counter that only grows between resets (the flags and barrier words are
-// cleared at the start of every call): the blocks of barrier k arrive as numbers k nb .. k nb + nb - 1 and leave
-// once the counter has reached (k + 1) nb.  The wait is bounded: false, with flags[11] set, when it gave up.
-__device__ __forceinline__ unsigned atomAddReleaseGpu(unsigned* p, unsigned v) {
-    unsigned old;
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
-}
-
-// The arrival is a release (it orders the block's writes before it, made the thread's own by the block barrier
-// ahead of it) and the wait an acquire load, so no separate fences are needed.
-__device__ __forceinline__ bool fftgBarrier(unsigned* bar, unsigned nb, int* flags) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        ok = 1;
-        const unsigned old = atomAddReleaseGpu(bar, 1u);
-        const unsigned target = (old / nb + 1) * nb;
-        if (old + 1 != target)
-            for (unsigned it = 0; (int) (ldAcquireGpu(bar) - target) < 0; it++)
-                if (it >= FFTG_SPIN_LIMIT) {
-                    ok = 0;
-                    atomicExch(flags + 11, 1);
-                    break;
-                }
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
 // Self-test of the bounded barrier wait: the launch's blocks wait at a barrier that expects one block more than
 // there are, so every wait runs out (FFTG_SPIN_LIMIT polls), sets flags[11] and returns.
 __global__ void k_barrier_probe(unsigned* bar, int* flags) { fftgBarrier(bar, gridDim.x + 1, flags); }
 
-// KC > 0: every grid of the launch is KC^3 (compile-time passes and index maps); 0: any grid.
-// ENERGY (the final pass): also the reciprocal energy (1/2) sum w G |F|^2 and its strain derivative, as k_conv
-// sums them, from the x-lines' spectrum before the product; block x writes conv partial x of its system and clears
-// partials x + K0, x + 2 K0, ... up to the system's convBlocks (the host requires K0 <= convBlocks).
-template <typename R, int KC, bool ENERGY = false>
-__global__ void __launch_bounds__(FftgThreads<R>::n) k_fft_grid(Dev dv, int gateDone) {
-    typedef typename CplxT<R>::T C;
-    const int s = blockIdx.y;
-    if ((gateDone & 1) && dv.scal[s * NSCAL + SC_DONE] != 0.0)
-        return;   // every block of the system
-    // gateDone & 2: the spread went to the fixed-point grid; its plane is converted (and cleared) on the load
-    long long* const fx = (gateDone & 2) ? dv.gridFix : nullptr;
-    const SysDev& S = dv.sys[s];
-    const int K0 = KC > 0 ? KC : S.K[0], K1 = KC > 0 ? KC : S.K[1], K2 = KC > 0 ? KC : S.K[2];
-    const int K2h = K2 / 2 + 1, P = (K1 + 1) / 2, ly = K1 + 1, lx = K0 + 1;
-    const int x = blockIdx.x;
-    if (x >= K0)
-        return;   // (a smaller grid than the launch's largest)
-    const int nline = K1 * K2h, lpb = (nline + K0 - 1) / K0, l0 = x * lpb;
-    const int nl = max(0, min(nline, l0 + lpb) - l0);
-    const int nT = blockDim.x, tid = threadIdx.x;
-    const float iK2 = __frcp_rn((float) K2), iK2h = __frcp_rn((float) K2h), iLpb = __frcp_rn((float) lpb);
-    // e / d: by a constant when the grid is one (the compiler multiplies), else through the float reciprocal
-    auto qd = [](int e, int d, float inv) { return KC > 0 ? e / d : fdiv(e, inv); };
-    extern __shared__ __align__(16) unsigned char smraw[];
-    C* W0 = (C*) smraw;
-    C* W1 = W0 + FFT_MAXK;
-    C* W2 = W1 + FFT_MAXK;
-    C* const b0 = W2 + FFT_MAXK;
-    C* const b1 = b0 + dv.fftgBuf;
-    const C* tw = (const C*) dv.twiddle;
-    for (int m = tid; m < K0; m += nT)
-        W0[m] = tw[S.twOff[0] + m];
-    for (int m = tid; m < K1; m += nT)
-        W1[m] = tw[S.twOff[1] + m];
-    for (int m = tid; m < K2; m += nT)
-        W2[m] = tw[S.twOff[2] + m];
-    R* const gx = (R*) dv.grid + S.gridOff + (size_t) x * K1 * K2;
-    C* const spec = (C*) dv.spec + S.specOff;
-    C* const plane = spec + (size_t) x * nline;
-    unsigned* const bar = dv.fftgBar + 2 * s;
-    // 1. plane x: rows 2p, 2p + 1 as one complex row [pair][z]; z; separation into y-lines [kz][y]; y
-    long long* const fxx = fx ? fx + S.gridOff + (size_t) x * K1 * K2 : nullptr;
-    for (int e = tid; e < P * K2; e += nT) {
-        const int pr = qd(e, K2, iK2), z = e - pr * K2;
-        C v;
-        if (fxx) {
-            v.x = (R) gridFixTake(fxx + 2 * pr * K2 + z);
-            v.y = (2 * pr + 1 < K1) ? (R) gridFixTake(fxx + (2 * pr + 1) * K2 + z) : (R) 0;
-        } else {
-            v.x = gx[2 * pr * K2 + z];
-            v.y = (2 * pr + 1 < K1) ? gx[(2 * pr + 1) * K2 + z] : (R) 0;
-        }
-        b0[e] = v;
-    }
-    __syncthreads();
-    C* Z = fftLinesK<R, -1, KC>(b0, b1, P, K2, K2, W2);
-    C* O = (Z == b0) ? b1 : b0;
-    for (int e = tid; e < P * K2h; e += nT) {
-        const int pr = qd(e, K2h, iK2h), kz = e - pr * K2h;
-        const C* zr = Z + pr * K2;
-        const C zk = zr[kz], zm = zr[kz == 0 ? 0 : K2 - kz];
-        C X, Y;   // X = (Z_k + conj Z_-k) / 2, Y = (Z_k - conj Z_-k) / 2i
-        X.x = (R) 0.5 * (zk.x + zm.x);
-        X.y = (R) 0.5 * (zk.y - zm.y);
-        Y.x = (R) 0.5 * (zk.y + zm.y);
-        Y.y = (R) 0.5 * (zm.x - zk.x);
-        C* o = O + kz * ly + 2 * pr;
-        o[0] = X;
-        if (2 * pr + 1 < K1)
-            o[1] = Y;
-    }
-    __syncthreads();
-    const C* F = fftLinesK<R, -1, KC>(O, Z, K2h, K1, ly, W1);
-    for (int e = tid; e < nline; e += nT) {
-        const int ky = qd(e, K2h, iK2h), kz = e - ky * K2h;
-        plane[e] = F[kz * ly + ky];
-    }
-    if (!fftgBarrier(bar, (unsigned) K0, dv.flags))
-        return;
-    // 2. my x-lines: forward along x, influence product, back
-    for (int e = tid; e < lpb * K0; e += nT) {   // consecutive threads: consecutive lines of a plane
-        const int xx = qd(e, lpb, iLpb), li = e - xx * lpb;
-        if (li < nl)
-            b0[li * lx + xx] = __ldcg(spec + (size_t) xx * nline + l0 + li);
-    }
-    __syncthreads();
-    C* Fx = fftLinesK<R, -1, KC>(b0, b1, nl, K0, lx, W0);
-    const R* infl = (const R*) dv.infl + S.specOff;
-    double acc[ENERGY ? NCONV : 1];
-#pragma unroll
-    for (int k = 0; k < (ENERGY ? NCONV : 1); k++)
-        acc[k] = 0.0;
-    const double fac = PI_D * PI_D / (S.beta * S.beta);
-    for (int e = tid; e < lpb * K0; e += nT) {
-        const int xx = qd(e, lpb, iLpb), li = e - xx * lpb;
-        if (li < nl) {
-            const R gk = infl[(size_t) xx * nline + l0 + li];
-            C& v = Fx[li * lx + xx];
-            if (ENERGY && (xx != 0 || l0 + li != 0)) {   // (the k = 0 term is left out, as k_conv does)
-                const int l = l0 + li, m3 = l % K2h, m2 = l / K2h, m1 = xx;
-                const double w = (m3 == 0 || ((K2 & 1) == 0 && m3 == K2 / 2)) ? 1.0 : 2.0;
-                const double nrm = (double) v.x * v.x + (double) v.y * v.y;
-                const double en = 0.5 * w * (double) gk * nrm;
-                acc[0] += en;
-                const double mm1 = (m1 <= K0 / 2) ? m1 : m1 - K0, mm2 = (m2 <= K1 / 2) ? m2 : m2 - K1, mm3 = m3;
-                double ms[3];
-#pragma unroll
-                for (int k = 0; k < 3; k++)
-                    ms[k] = mm1 * S.recip[3 * k] + mm2 * S.recip[3 * k + 1] + mm3 * S.recip[3 * k + 2];
-                const double m2s = ms[0] * ms[0] + ms[1] * ms[1] + ms[2] * ms[2];
-                const double c2 = 2.0 * (fac + 1.0 / m2s);
-#pragma unroll
-                for (int a = 0; a < 3; a++)
-#pragma unroll
-                    for (int b = 0; b < 3; b++)
-                        acc[ENERGY ? 1 + 3 * a + b : 0] += en * ((a == b ? -1.0 : 0.0) + c2 * ms[a] * ms[b]);
-            }
-            v.x *= gk;
-            v.y *= gk;
-        }
-    }
-    if (ENERGY) {
-        blockReduce<NCONV>(acc, 0u);
-        if (tid == 0)
-            for (int k = 0; k < NCONV; k++)
-                dv.convPartial[(size_t) (dv.convPartialOff[s] + x) * NCONV + k] = acc[k];
-        if (tid < NCONV * 16)
-            for (int b = x + K0 * (1 + tid / NCONV); b < S.convBlocks; b += 16 * K0)
-                dv.convPartial[(size_t) (dv.convPartialOff[s] + b) * NCONV + tid % NCONV] = 0.0;
-    }
-    __syncthreads();
-    const C* Gx = fftLinesK<R, 1, KC>(Fx, Fx == b0 ? b1 : b0, nl, K0, lx, W0);
-    for (int e = tid; e < lpb * K0; e += nT) {
-        const int xx = qd(e, lpb, iLpb), li = e - xx * lpb;
-        if (li < nl)
-            spec[(size_t) xx * nline + l0 + li] = Gx[li * lx + xx];
-    }
-    if (!fftgBarrier(bar, (unsigned) K0, dv.flags))
-        return;
-    // 3. plane x back: y-lines [kz][y]; y; two real rows from one complex row; z
-    for (int e = tid; e < nline; e += nT) {
-        const int ky = qd(e, K2h, iK2h), kz = e - ky * K2h;
-        b0[kz * ly + ky] = __ldcg(plane + e);
-    }
-    __syncthreads();
-    C* Gy = fftLinesK<R, 1, KC>(b0, b1, K2h, K1, ly, W1);
-    C* O2 = (Gy == b0) ? b1 : b0;
-    for (int e = tid; e < P * K2; e += nT) {
-        const int pr = qd(e, K2, iK2), k = e - pr * K2;
-        const bool upper = k >= K2h;
-        const int kk = upper ? K2 - k : k;
-        const bool realOnly = (k == 0) || ((K2 & 1) == 0 && k == K2 / 2);
-        const C* gy = Gy + kk * ly + 2 * pr;
-        C X = gy[0], Y;
-        Y.x = 0;
-        Y.y = 0;
-        if (2 * pr + 1 < K1)
-            Y = gy[1];
-        if (upper) {
-            X.y = -X.y;
-            Y.y = -Y.y;
-        }
-        if (realOnly) {
-            X.y = 0;
-            Y.y = 0;
-        }
-        C Zv;   // X + i Y
-        Zv.x = X.x - Y.y;
-        Zv.y = X.y + Y.x;
-        O2[e] = Zv;
-    }
-    __syncthreads();
-    const C* Zt = fftLinesK<R, 1, KC>(O2, Gy, P, K2, K2, W2);
-    for (int e = tid; e < P * K2; e += nT) {
-        const int pr = qd(e, K2, iK2), z = e - pr * K2;
-        gx[2 * pr * K2 + z] = Zt[e].x;
-        if (2 * pr + 1 < K1)
-            gx[(2 * pr + 1) * K2 + z] = Zt[e].y;
-    }
-}
+// ------------------------------------------------------------------------------------------------ interpolation
 
 // Interpolation from the potential grid: f_a = sum (d theta_a) theta theta phi (the field, E_rec = -sum_a K_a
 // recip[:, a] f_a, core/pgm_core.cpp:241-264); FINAL also the second derivatives, the potential and the
@@ -2271,19 +1910,6 @@ __global__ void __launch_bounds__(256) k_gvdw(Dev dv) {
 }
 
 // ------------------------------------------------------------------------------------------------ CG
-
-// The initial guess x0 of component g = 3 gi + k when it does not depend on b (guess 1: zero; 2: history slot;
-// 3: mu3 from history; 4: mu4 from history) (core/pgm_core.cpp:309-329).
-__device__ __forceinline__ double historyGuess(const Dev& dv, int guess, size_t g, size_t hs) {
-    const int h0 = dv.ctl->h[0], h1 = dv.ctl->h[1], h2 = dv.ctl->h[2], h3 = dv.ctl->h[3];
-    switch (guess) {
-    case 1: return 0.0;
-    case 2: return dv.hist[h0 * hs + g];
-    case 3: return 3 * dv.hist[h0 * hs + g] - 3 * dv.hist[h1 * hs + g] + dv.hist[h2 * hs + g];
-    default:
-        return 4 * dv.hist[h0 * hs + g] - 6 * dv.hist[h1 * hs + g] + 4 * dv.hist[h2 * hs + g] - dv.hist[h3 * hs + g];
-    }
-}
 
 // x0 of a predicted step before the permanent field (guess >= 1), so that one pair sweep forms E_perm and T x0
 // together; k_cg_b then writes the same x0 again.

@@ -24,7 +24,7 @@
 // reports the evaluation as failed.
 #pragma once
 
-#include "kernels.cuh"
+#include "gridfft.cuh"
 
 namespace pgmb200 {
 
@@ -251,13 +251,8 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_BLOCKS_PER_SM) k_cg_persisten
         return;   // converged at the initial guess (every block alike)
     const int n = dv.nAtoms, nb = gridDim.x, tid = threadIdx.x, nT = blockDim.x;
     const int K0 = KC > 0 ? KC : S.K[0], K1 = KC > 0 ? KC : S.K[1], K2 = KC > 0 ? KC : S.K[2];
-    const int K2h = K2 / 2 + 1, NP = (K1 + 1) / 2, ly = K1 + 1, lx = K0 + 1;
     const int x = blockIdx.x;
     const bool planeBlock = x < K0;
-    const int nline = K1 * K2h, lpb = (nline + K0 - 1) / K0, l0 = x * lpb;
-    const int nl = planeBlock ? max(0, min(nline, l0 + lpb) - l0) : 0;
-    const float iK2 = __frcp_rn((float) K2), iK2h = __frcp_rn((float) K2h), iLpb = __frcp_rn((float) lpb);
-    auto qd = [](int e, int d, float inv) { return KC > 0 ? e / d : fdiv(e, inv); };
     unsigned* const gbar = dv.pcgBar;        // every block
     unsigned* const pbar = dv.pcgBar + 1;    // the plane blocks
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -275,8 +270,9 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_BLOCKS_PER_SM) k_cg_persisten
         for (int m = tid; m < K2; m += nT)
             W2[m] = tw[S.twOff[2] + m];
     }
+    const PlaneFft<float, KC> fft(K0, K1, K2, b0, b1, W0, W1, W2);
+    const int nline = fft.nline, l0 = x * fft.lpb, nl = min(nline, l0 + fft.lpb) - l0;
     C* const spec = (C*) dv.spec + S.specOff;
-    C* const myPlane = spec + (size_t) x * nline;
     double* const part = dv.pcgPartial;
     // the slot-group phases (spread, gather): the groups' shared spline rows, the fixed-point charge grid and the
     // float potential grid
@@ -323,114 +319,29 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_BLOCKS_PER_SM) k_cg_persisten
             return;
         // ---- F: the plane blocks' reciprocal part, the other blocks' direct part
         if (planeBlock) {
-            // plane x from the fixed-point grid (cleared for the next spread): rows 2p, 2p + 1 as one complex row
-            // [pair][z]; z; separation into y-lines [kz][y]; y
+            // plane x from the fixed-point grid (cleared for the next spread), its share of the x-lines with the
+            // influence product, and back into the potential grid
             long long* const fxx = gfix + (size_t) x * K1 * K2;
-            auto take = [](long long* g) {
-                const long long v = __ldcg(g);
-                __stcg(g, 0ll);
-                return (float) ((double) v * (1.0 / 4294967296.0));
-            };
-            for (int e = tid; e < NP * K2; e += nT) {
-                const int pr = qd(e, K2, iK2), z = e - pr * K2;
-                C v;
-                v.x = take(fxx + 2 * pr * K2 + z);
-                v.y = (2 * pr + 1 < K1) ? take(fxx + (2 * pr + 1) * K2 + z) : 0.f;
-                b0[e] = v;
-            }
-            __syncthreads();
-            C* Z = fftLinesK<float, -1, KC>(b0, b1, NP, K2, K2, W2);
-            C* O = (Z == b0) ? b1 : b0;
-            for (int e = tid; e < NP * K2h; e += nT) {
-                const int pr = qd(e, K2h, iK2h), kz = e - pr * K2h;
-                const C* zr = Z + pr * K2;
-                const C zk = zr[kz], zm = zr[kz == 0 ? 0 : K2 - kz];
-                C X, Y;
-                X.x = 0.5f * (zk.x + zm.x);
-                X.y = 0.5f * (zk.y - zm.y);
-                Y.x = 0.5f * (zk.y + zm.y);
-                Y.y = 0.5f * (zm.x - zk.x);
-                C* o = O + kz * ly + 2 * pr;
-                o[0] = X;
-                if (2 * pr + 1 < K1)
-                    o[1] = Y;
-            }
-            __syncthreads();
-            const C* F = fftLinesK<float, -1, KC>(O, Z, K2h, K1, ly, W1);
-            for (int e = tid; e < nline; e += nT) {
-                const int ky = qd(e, K2h, iK2h), kz = e - ky * K2h;
-                myPlane[e] = F[kz * ly + ky];
-            }
+            fft.forward(
+                [&](int e) {
+                    const long long v = __ldcg(fxx + e);
+                    __stcg(fxx + e, 0ll);
+                    return (float) ((double) v * (1.0 / 4294967296.0));
+                },
+                spec + (size_t) x * nline);
             if (!fftgBarrier(pbar, (unsigned) K0, dv.flags))
                 return;
-            // my x-lines: forward along x, influence product, back
-            for (int e = tid; e < lpb * K0; e += nT) {
-                const int xx = qd(e, lpb, iLpb), li = e - xx * lpb;
-                if (li < nl)
-                    b0[li * lx + xx] = __ldcg(spec + (size_t) xx * nline + l0 + li);
-            }
-            __syncthreads();
-            C* Fx = fftLinesK<float, -1, KC>(b0, b1, nl, K0, lx, W0);
             const float* infl = (const float*) dv.infl + S.specOff;
-            for (int e = tid; e < lpb * K0; e += nT) {
-                const int xx = qd(e, lpb, iLpb), li = e - xx * lpb;
-                if (li < nl) {
-                    const float gk = infl[(size_t) xx * nline + l0 + li];
-                    C& v = Fx[li * lx + xx];
-                    v.x *= gk;
-                    v.y *= gk;
-                }
-            }
-            __syncthreads();
-            const C* Gx = fftLinesK<float, 1, KC>(Fx, Fx == b0 ? b1 : b0, nl, K0, lx, W0);
-            for (int e = tid; e < lpb * K0; e += nT) {
-                const int xx = qd(e, lpb, iLpb), li = e - xx * lpb;
-                if (li < nl)
-                    spec[(size_t) xx * nline + l0 + li] = Gx[li * lx + xx];
-            }
+            fft.lines(spec, l0, nl, [&](int m1, int l, C v) {
+                const float gk = infl[(size_t) m1 * nline + l];
+                v.x *= gk;
+                v.y *= gk;
+                return v;
+            });
             if (!fftgBarrier(pbar, (unsigned) K0, dv.flags))
                 return;
-            // plane x back: y-lines; y; two real rows from one complex row; z
-            for (int e = tid; e < nline; e += nT) {
-                const int ky = qd(e, K2h, iK2h), kz = e - ky * K2h;
-                b0[kz * ly + ky] = __ldcg(myPlane + e);
-            }
-            __syncthreads();
-            C* Gy = fftLinesK<float, 1, KC>(b0, b1, K2h, K1, ly, W1);
-            C* O2 = (Gy == b0) ? b1 : b0;
-            for (int e = tid; e < NP * K2; e += nT) {
-                const int pr = qd(e, K2, iK2), k = e - pr * K2;
-                const bool upper = k >= K2h;
-                const int kk = upper ? K2 - k : k;
-                const bool realOnly = (k == 0) || ((K2 & 1) == 0 && k == K2 / 2);
-                const C* gy = Gy + kk * ly + 2 * pr;
-                C X = gy[0], Y;
-                Y.x = 0.f;
-                Y.y = 0.f;
-                if (2 * pr + 1 < K1)
-                    Y = gy[1];
-                if (upper) {
-                    X.y = -X.y;
-                    Y.y = -Y.y;
-                }
-                if (realOnly) {
-                    X.y = 0.f;
-                    Y.y = 0.f;
-                }
-                C Zv;
-                Zv.x = X.x - Y.y;
-                Zv.y = X.y + Y.x;
-                O2[e] = Zv;
-            }
-            __syncthreads();
-            const C* Zt = fftLinesK<float, 1, KC>(O2, Gy, NP, K2, K2, W2);
             float* const gx = gpot + (size_t) x * K1 * K2;   // plane x of the potential
-            for (int e = tid; e < NP * K2; e += nT) {
-                const int pr = qd(e, K2, iK2), z = e - pr * K2;
-                gx[2 * pr * K2 + z] = Zt[e].x;
-                if (2 * pr + 1 < K1)
-                    gx[(2 * pr + 1) * K2 + z] = Zt[e].y;
-            }
+            fft.inverse(spec + (size_t) x * nline, [&](int e, float v) { gx[e] = v; });
         } else {
             const int groups = nT / GS;
             pcgPairField<GS, PASS == 2>(dv, (x - K0) * groups + tid / GS, (nb - K0) * groups);
