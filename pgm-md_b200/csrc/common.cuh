@@ -471,10 +471,11 @@ constexpr float GRID_FIX_SCALE = 4294967296.0f;   // 2^32
 __device__ __forceinline__ void gridFixAdd(long long* g, float v) {
     atomicAdd((unsigned long long*) g, (unsigned long long) __float2ll_rn(v * GRID_FIX_SCALE));
 }
+__device__ __forceinline__ float gridFixValue(long long v) { return (float) ((double) v * (1.0 / 4294967296.0)); }
 __device__ __forceinline__ float gridFixTake(long long* g) {   // the value, and the word cleared for the next spread
     const long long v = *g;
     *g = 0;
-    return (float) ((double) v * (1.0 / 4294967296.0));
+    return gridFixValue(v);
 }
 
 // The initial guess x0 of component g = 3 gi + k when it does not depend on b (guess 1: zero; 2: history slot;

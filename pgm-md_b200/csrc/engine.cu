@@ -1261,8 +1261,7 @@ struct Engine::Impl {
     // whether the field passes' spread (launchSpread) writes the fixed-point grid: the warp-per-atom kernel only
     bool spreadFix() const { return fixMode() && !planesMode() && !linesMode() && !tilesMode(); }
     void gridFromFix(cudaStream_t sm, const Dev& d) {
-        const int blocks = (int) std::min<long long>((gridTotal + 255) / 256, 4 * 148);
-        k_grid_from_fix<<<blocks, 256, 0, sm>>>(d);
+        k_grid_from_fix<<<(unsigned) ((gridTotal + 1023) / 1024), 256, 0, sm>>>(d);
         CU(cudaGetLastError());
     }
 

@@ -13,11 +13,21 @@
 
 namespace pgmb200 {
 
-// The fixed-point grid to the float grid (every point), clearing the fixed-point grid.
-__global__ void k_grid_from_fix(Dev dv) {
-    const size_t n = (size_t) dv.gridTotal, stride = (size_t) gridDim.x * blockDim.x;
-    for (size_t k = (size_t) blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride)
-        ((float*) dv.grid)[k] = gridFixTake(dv.gridFix + k);
+// The fixed-point grid to the float grid (every point), clearing the fixed-point grid: four points per thread and no
+// loop, since a walk whose every step waits for its load is bound by latency (592 blocks walking 8.0 M points of a
+// 1024-box batch took 463 us, 1.1 M points of a 104^3 grid 53 us; the bytes, 20 a point, take 25 and 3.5 us).
+__global__ void __launch_bounds__(256) k_grid_from_fix(Dev dv) {
+    const size_t n = (size_t) dv.gridTotal, k = 4 * ((size_t) blockIdx.x * blockDim.x + threadIdx.x);
+    if (k + 4 <= n) {
+        const longlong2 a = *(const longlong2*) (dv.gridFix + k), b = *(const longlong2*) (dv.gridFix + k + 2);
+        *(longlong2*) (dv.gridFix + k) = make_longlong2(0, 0);
+        *(longlong2*) (dv.gridFix + k + 2) = make_longlong2(0, 0);
+        *(float4*) ((float*) dv.grid + k) = make_float4(gridFixValue(a.x), gridFixValue(a.y), gridFixValue(b.x),
+                                                        gridFixValue(b.y));
+    } else {
+        for (size_t j = k; j < n; j++)
+            ((float*) dv.grid)[j] = gridFixTake(dv.gridFix + j);
+    }
 }
 
 // Block-wide compaction of the systems still iterating (scal[DONE] == 0) into actSys / actOff / actCount, in
