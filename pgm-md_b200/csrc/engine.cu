@@ -199,6 +199,7 @@ struct Engine::Impl {
     int pcgBlocks = 0;         // its blocks (one per SM)
     size_t pcgSmem = 0;
     int fftcBuf = 0, fftcC = 16, fftgBuf = 0, maxK0 = 0;
+    int pcgKc = 0;             // the one system's grid is pcgKc^3, or 0
     int fftgKc = 0;            // the grid transforms' compile-time size (every grid fftgKc^3), or 0
     size_t fftgSmem = 0;
     int maxLineBlocks = 0;
@@ -644,6 +645,7 @@ struct Engine::Impl {
             for (int k = 0; k < nsys; k++)
                 for (int a = 0; a < 3; a++)
                     fftgKc = sysK[k][a] == fftgKc ? fftgKc : 0;
+            pcgKc = fftgKc;
             if (fftgKc != 32 && fftgKc != 40 && fftgKc != 48 && fftgKc != 64)
                 fftgKc = 0;
         }
@@ -1207,18 +1209,18 @@ struct Engine::Impl {
         CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, devId));
         CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, devId));
         const int* K = sysK[0].data();
-        pcgSmem = (3 * (size_t) FFT_MAXK + 2 * (size_t) fftgBuf) * 8;
-        if (!coop || pcgSmem > (size_t) optin || K[0] + PCG_MIN_PAIR_BLOCKS > sms)
+        pcgBlocks = std::min(sms, PCG_MAX_BLOCKS);   // (one per SM; the plane blocks are 0 .. K0-1)
+        pcgSmem = pcgSmemBytes((n + pcgBlocks - 1) / pcgBlocks, fftgBuf);
+        if (!coop || pcgSmem > (size_t) optin || K[0] + PCG_MIN_PAIR_BLOCKS > pcgBlocks)
             return;
-        PcgKernel kfn = persistentKernel(pairGS);
+        PcgKernel kfn = pcgKernel(pcgKc);
         CU(cudaFuncSetAttribute((const void*) kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) pcgSmem));
         int perSm = 0;
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kfn, PCG_THREADS, pcgSmem));
         if (perSm < 1)
             return;
-        pcgBlocks = sms * std::min(perSm, PCG_BLOCKS_PER_SM);   // (the plane blocks, 0 .. K0-1, one per SM)
         pcgOk = true;
-        dPcgPartial.ensure((size_t) 2 * pcgBlocks * 4 * 8);
+        dPcgPartial.ensure((size_t) pcgBlocks * 5 * 8);
     }
 
     // The plane-owner spread and gather: mixed precision, one system, order 6; tiles of PL_YCH rows (+ 5 halo
@@ -1360,12 +1362,10 @@ struct Engine::Impl {
         CU(cudaGetLastError());
     }
 
-    PcgKernel persistentKernel(int lanes, int pass = 0) { return pcgKernel(lanes, fftgKc, pass); }
-
-    // The whole CG loop (pass 0), or one field pass of the dipoles vec (1) and the charges (2): one cooperative
-    // launch of the persistent kernel (one block per SM).
-    void launchPersistent(cudaStream_t sm, const Dev& d, int pass = 0, const double* vec = nullptr) {
-        PcgKernel kfn = persistentKernel(pairGS, pass);
+    // The whole CG solve after the permanent field (or for the right-hand side in b): one cooperative launch of the
+    // persistent kernel (one block per SM).
+    void launchPersistent(cudaStream_t sm, const Dev& d) {
+        PcgKernel kfn = pcgKernel(pcgKc);
         CU(cudaFuncSetAttribute((const void*) kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) pcgSmem));
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[1];
@@ -1379,7 +1379,11 @@ struct Engine::Impl {
         cfg.numAttrs = 1;
         Dev dp = d;   // (its spread always goes to the fixed-point grid)
         dp.gridFix = dGridFix.as<long long>();
-        CU(cudaLaunchKernelEx(&cfg, kfn, dp, planeNyc, vec));
+        // the rows of the pair pass that a plane block's transforms are worth, from the expected length of a row
+        const SysDev& S = sysHost[0];
+        const double row = std::max(1.0, 4.0 / 3.0 * PI_D * S.cutoff * S.cutoff * S.cutoff * (n / S.volume));
+        const int planeSlots = (int) std::min((double) n, PCG_PLANE_PAIRS / row);
+        CU(cudaLaunchKernelEx(&cfg, kfn, dp, planeSlots));
     }
 
     bool persistentMode() const { return tfMode == TF_PCG; }
@@ -1692,7 +1696,7 @@ struct Engine::Impl {
             // the permanent field's PME half (main stream).  Without a skin, on the plain first pass, the record
             // kernel also forms the permanent field's direct part (after the permanent spread wrote the sources),
             // in place of a pair pass of its own.
-            const bool pcg = std::is_same<R, float>::value && persistentMode();
+            const bool pcg = std::is_same<R, float>::value && persistentMode() && !refining();
             if (!dualFirstPass()) {
                 // the permanent field's PME half on the side stream, whose higher priority lets the cooperative grid
                 // kernel's blocks in ahead of the list build's; on the main stream the list's rows and then the
@@ -1721,14 +1725,10 @@ struct Engine::Impl {
                     pairField<R, true>(sm, d, 0);
                 }
                 CU(cudaStreamWaitEvent(sm, evJoin, 0));
+                if (pcg)   // the solve from here on is the persistent kernel's
+                    return;
                 k_cg_b<<<(int) chunkSys.size(), CHUNK, 0, sm>>>(d);
                 CU(cudaGetLastError());
-                if (pcg) {   // A x0 as one pass of the persistent kernel, then the loop's set-up
-                    launchPersistent(sm, d, 1, d.x);
-                    k_cg_init<<<(int) chunkSys.size(), CHUNK, 0, sm>>>(d);
-                    CU(cudaGetLastError());
-                    return;
-                }
                 CU(cudaMemsetAsync(d.grid, 0, gridTotal * realSize(), sm));
                 fieldPass<R, false>(sm, sd, d, 1, d.x, false);
                 k_cg_init<<<(int) chunkSys.size(), CHUNK, 0, sm>>>(d);
@@ -2769,6 +2769,13 @@ int Engine::Impl::solveDevice(double tol) {
     auto run = [&](auto tag) {
         typedef decltype(tag) R;
         CU(cudaMemsetAsync(d.flags, 0, flagBytes(), st));
+        if (persistentMode()) {
+            launchPersistent(st, d);
+            CU(cudaMemcpyAsync(hFlags, d.flags, 16 * sizeof(int), cudaMemcpyDeviceToHost, st));
+            CU(cudaStreamSynchronize(st));
+            barrierCheck();
+            return;
+        }
         k_cg_b<<<(int) chunkSys.size(), CHUNK, 0, st>>>(d);
         CU(cudaMemsetAsync(d.grid, 0, gridTotal * realSize(), st));
         fieldPass<R, false>(st, side, d, 1, d.x, false);
@@ -2934,6 +2941,13 @@ int Engine::solve(const double* rhs, double* x, double tol) {
     auto run = [&](auto tag) {
         typedef decltype(tag) R;
         CU(cudaMemsetAsync(d.flags, 0, I.flagBytes(), I.st));
+        if (I.persistentMode()) {
+            I.launchPersistent(I.st, d);
+            CU(cudaMemcpyAsync(I.hFlags, d.flags, 16 * sizeof(int), cudaMemcpyDeviceToHost, I.st));
+            CU(cudaStreamSynchronize(I.st));
+            I.barrierCheck();
+            return;
+        }
         k_cg_b<<<(int) I.chunkSys.size(), CHUNK, 0, I.st>>>(d);
         CU(cudaMemsetAsync(d.grid, 0, I.gridTotal * I.realSize(), I.st));
         I.fieldPass<R, false>(I.st, I.side, d, 1, d.x, false);
@@ -2988,8 +3002,8 @@ int Engine::kernelLaunches() const {
         it = std::max(it, (int) I.lastResults[(size_t) k * NRES + 14]);
     const int fp = 4;
     const int perIt = fp + (I.nsys == 1 && I.fuseCgA ? 1 : 2);   // single system: A p in the gather
-    if (I.persistentMode() && I.s.polarizable)   // the bins and one persistent launch for the whole loop
-        return 7 + (I.lastBuilt ? 5 : 0) + 2 * fp + 2 + 2 + 7 + (I.gvdwOn ? 1 : 0);
+    if (I.persistentMode() && I.s.polarizable)   // the permanent field's pass and one launch for the whole solve
+        return 7 + (I.lastBuilt ? 5 : 0) + fp + 1 + 7 + (I.gvdwOn ? 1 : 0);
     return 7 + (I.lastBuilt ? 5 : 0) + (I.s.polarizable ? 2 * fp + 2 + perIt * it : 0) + 7 + (I.gvdwOn ? 1 : 0);
 }
 

@@ -1,25 +1,33 @@
 // The CG solve of one system in mixed precision as ONE persistent cooperative kernel (one block per SM), for
-// grids whose dimensions have at most FFT_MAXK points and the prime factors 2, 3, 5.
+// grids whose dimensions have at most FFT_MAXK points and the prime factors 2, 3, 5: the right-hand side, the initial
+// guess, A x0, every iteration of core/pgm_core.cpp:297-385 (A v = v/alpha - T v; T v = pair + reciprocal + self field)
+// and the convergence test, with barriers of the launch's blocks in place of kernel boundaries and graph nodes.
 //
-// Every CG iteration of core/pgm_core.cpp:351-385 (A v = v/alpha - T v; T v = pair + reciprocal + self field)
-// runs inside the kernel, with grid barriers between its phases instead of kernel boundaries and graph nodes:
+// A block owns a run of slots.  Their x, r, p, A p, alpha and spline coefficients stay in its shared memory from the
+// first pass to the last, so an iteration meets global memory only where blocks exchange data:
 //
-//   S  (every block, 8 lanes per slot of its chunk)  p = z + beta p; the pair pass's float copy of p; the PME
-//      weights (q, e_a = K_a p . recip[:, a]) and the spread of the atom into the 64-bit fixed-point grid
-//      (global atomics, the same points and arithmetic as k_spread; integer sums do not depend on their order,
-//      so the solve repeats bit for bit);                                                         grid barrier
-//   F  blocks 0 .. K0-1 own the x-planes of the PME grid: the plane is read from the fixed-point grid (and
-//      cleared for the next spread), transformed along z and y, the x-lines exchanged through L2 (two barriers
-//      of the plane blocks), the influence product, transformed back and stored to the potential grid.
-//      Blocks K0 .. end run the direct-space field pass of the iteration's direction over the pair records.
-//                                                                                                  grid barrier
-//   G  (every block, 8 lanes per slot of its chunk) E_rec at the atom from the potential grid, the atom's row of
-//      A p and the block's share of p . A p;                                                        grid barrier
-//   U  (every block) alph from the shares (fixed order), x, r, z of its slots, shares of z'.(r' - r), r'.z',
-//      max |z'|;                                                                                    grid barrier
-//   C  (every block, identically) beta, rz, err, the iteration count and the convergence test.
+//   S  (every block, 16 lanes per slot) the direction's float copy for the pair pass, its PME weights (q, e_a = K_a p .
+//      recip[:, a]) and the spread into the 64-bit fixed-point grid (global atomics, the points and arithmetic of
+//      k_spread; integer sums do not depend on their order, so the solve repeats bit for bit);      grid barrier
+//   F  blocks 0 .. K0-1 own the x-planes of the PME grid: the plane is read from the fixed-point grid (and cleared for
+//      the next spread), transformed, its share of the x-lines multiplied by the influence function (two barriers of
+//      the plane blocks; linefft.cuh) and transformed back into the potential grid.  The others run the
+//      direct-space field pass of the direction over the pair records (the plane blocks join in when there are many).                                grid barrier
+//   G  (every block, 16 lanes per slot) E_rec at the atom from the potential grid, the atom's row of A p and the block's
+//      shares of p . A p, z . A p and A p . alpha A p;                                                grid barrier
+//   U  (every block, its own slots) alph = rz / p.Ap, r' = r - alph A p, z' = alpha r'.  The next direction's beta
+//      follows from the same sums, z'.(r' - r) = -alph (z.Ap - alph Ap.alpha Ap), so it needs no exchange of its own
+//      and U runs into the next S.  r'.z', which the next alph needs, and max |z'|, which the convergence test needs,
+//      go around with the next S's barrier (a recurrence for r'.z' would keep the rounding of the first one); the
+//      spread of the iteration after the last is then dropped (the plane blocks clear it).
 //
-// Every reduction sums in a fixed order.  Data other blocks wrote in this launch is read past L1 (__ldcg).
+// What bounds it (8550 atoms, 48^3, one B200): the chain of phases and barriers, in us an iteration S 4.7, F 13.5 (the pair
+// pass's 61 MB of records through L2 on 100 SMs; the plane blocks take 10), G 3.2, U with its sums 2.7, barriers 9.  With
+// p, x, r in global memory, a barrier more, the pair pass's sources read past L1 and 512 threads, an evaluation of ten
+// iterations took 691 us against 593.
+//
+// Every reduction sums in a fixed order.  The barriers' acquire makes what other blocks wrote visible to plain loads, so
+// the pair pass's gathers and the stencil's reads share lines through L1.
 // Barrier waits are bounded (about a second); a block that gives up sets flags[11] and returns, and the host
 // reports the evaluation as failed.
 #pragma once
@@ -28,10 +36,17 @@
 
 namespace pgmb200 {
 
-constexpr int PCG_THREADS = 512;
+// 1024 threads (64 registers): the pair pass keeps 98 KB of records in flight per SM; with 512 threads it took 17.2 us
+// (8550 atoms) where 1024 take 13.
+constexpr int PCG_THREADS = 1024;
+constexpr int PCG_MAX_BLOCKS = 160;          // the totals' loads are unrolled for at most this many blocks
 constexpr int PCG_MIN_PAIR_BLOCKS = 16;      // blocks left for the pair pass beside the plane blocks
-constexpr int PCG_SLOT_LANES = 8;            // lanes per slot in the spread and gather phases
-constexpr int PCG_BLOCKS_PER_SM = 1;         // resident blocks per SM (two, at 64 registers, measured slower)
+constexpr int PCG_SLOT_LANES = 16;           // lanes per slot in the spread and gather phases
+// Directed pairs that a block sums while a plane block transforms its plane (9.9 us at 48^3): the plane blocks take
+// that many fewer of the pair pass's rows, if any.
+constexpr int PCG_PLANE_PAIRS = 32000;
+constexpr int PCG_SPL = 40;                  // floats per slot of the spline rows: theta, dtheta [3][6], padded so that
+                                             // the four slots of a warp read different banks
 
 // The spline record of one atom of the plane-owner kernels' bins (order P): its slot, b1, b2 and b0 mod K0, and
 // theta and dtheta of the three dimensions, c[dim 2P + kind P + j].
@@ -40,227 +55,138 @@ template <int P> struct PmeRec {
     float c[6 * P];
 };
 
-// The spread of slot s (its atom's weights w = (q, e0, e1, e2)) into the 64-bit fixed-point grid by a group of L
-// lanes (lane hl, mask `mask`, shared rows `row` for the evaluation's spline coefficients): a stencil column
-// (j2, j3) per lane and round, a loop over j1; the groups of a warp keep several atoms' loads and atomics in
-// flight.  The points and per-point arithmetic of k_spread, so both add the same integers.
-// The group's share of slot s's spline coefficients (k = hl, hl + L, ...) and base index (lanes hl < 3), loaded
-// ahead of the direction update that the spread waits for.
-template <int P, int L> struct SpreadPre {
-    float c[(6 * P + L - 1) / L];
-    int bl;
-    __device__ __forceinline__ void load(const Dev& dv, int s, int i, int hl) {
-        const float* sp = (const float*) dv.spl + (size_t) s * 9 * MAXP;
-#pragma unroll
-        for (int m = 0; m < (6 * P + L - 1) / L; m++) {
-            const int k = hl + m * L;
-            if (k < 6 * P) {
-                const int kind = k / (3 * P), dim = (k / P) % 3, j = k % P;
-                c[m] = sp[(kind * 3 + dim) * MAXP + j];
-            }
-        }
-        bl = hl < 3 ? dv.pmeBase[3 * i + hl] : 0;
-    }
-};
-
-template <int P, int L>
-__device__ __forceinline__ void pcgSpreadHalf(const Dev& dv, const SysDev& S, long long* gfix, float4 w,
-                                             const SpreadPre<P, L>& pre, float (*sth)[3][P], float (*sdth)[3][P],
-                                             int row, int hl, unsigned mask) {
-#pragma unroll
-    for (int m = 0; m < (6 * P + L - 1) / L; m++) {
-        const int k = hl + m * L;
-        if (k < 6 * P) {
-            const int kind = k / (3 * P), dim = (k / P) % 3, j = k % P;
-            if (kind == 0)
-                sth[row][dim][j] = pre.c[m];
-            else
-                sdth[row][dim][j] = pre.c[m];
-        }
-    }
-    const int bl = pre.bl;
-    const int b0 = __shfl_sync(mask, bl, 0, L), b1 = __shfl_sync(mask, bl, 1, L), b2 = __shfl_sync(mask, bl, 2, L);
-    __syncwarp(mask);
-    const float qr = w.x, e0 = w.y, e1 = w.z, e2 = w.w;
-    const int K0 = S.K[0], K1 = S.K[1], K2 = S.K[2];
-    const size_t plane = (size_t) K1 * K2;
-    for (int c = hl; c < P * P; c += L) {
-        const int j2 = c / P, j3 = c % P;
-        const float t2 = sth[row][1][j2], u2 = sdth[row][1][j2];
-        const float t3 = sth[row][2][j3], u3 = sdth[row][2][j3];
-        const float c23 = t2 * t3;
-        const float a = qr * c23 + e1 * u2 * t3 + e2 * t2 * u3;
-        const float b = e0 * c23;
-        const size_t col = (size_t) wrapIndex(b1 - j2, K1) * K2 + wrapIndex(b2 - j3, K2);
-#pragma unroll
-        for (int j1 = 0; j1 < P; j1++)
-            gridFixAdd(gfix + col + (size_t) wrapIndex(b0 - j1, K0) * plane,
-                       (float) (a * sth[row][0][j1] + b * sdth[row][0][j1]));
-    }
-    __syncwarp(mask);   // (the next slot of this group overwrites the shared rows)
+// Shared memory of a block of `per` slots beside the transforms' tables and buffers (fftgBuf complex elements each).
+__host__ __device__ inline size_t pcgSmemBytes(int per, int fftgBuf) {
+    return (3 * (size_t) FFT_MAXK + 2 * (size_t) fftgBuf) * sizeof(float2) + (size_t) per * (13 * 8 + PCG_SPL * 4 + 4 * 4);
 }
 
-// E_rec at the atom of slot s from the potential grid gpot (written by other blocks in this launch: read past
-// L1) by a group of L lanes (as pcgSpreadHalf): f_a = sum (d theta_a) theta theta phi over the stencil, E_rec =
-// -sum_a K_a recip[:, a] f_a (core/pgm_core.cpp:241-264), the lanes' sums in double; or (CGA, the CG iterations)
-// instead the atom's row of A p = p / alpha - (E_pair + E_rec + cs p) (core/pgm_core.cpp:363) and the returned
-// share p_k (A p)_k of lanes hl = k < 3 (0 elsewhere).
-template <int P, bool CGA, int L>
-__device__ __forceinline__ double pcgGatherHalf(const Dev& dv, const SysDev& S, const float* gpot, int s,
-                                               float (*sth)[3][P], float (*sdth)[3][P], int row, int hl,
-                                               unsigned mask, double cs) {
-    const int i = dv.slotAtom[s];
-    double alI = 0.0, pI = 0.0, eI = 0.0;   // (CGA) the inputs of the atom's A p row, loaded first
-    if (CGA && hl < 3) {
-        alI = dv.alpha[i];
-        pI = dv.p[3 * i + hl];
-        eI = __ldcg(dv.Epair + 3 * i + hl);
-    }
-    const float* sp = (const float*) dv.spl + (size_t) s * 9 * MAXP;
-    for (int k = hl; k < 6 * P; k += L) {
-        const int kind = k / (3 * P), dim = (k / P) % 3, j = k % P;
-        const float v = sp[(kind * 3 + dim) * MAXP + j];
-        if (kind == 0)
-            sth[row][dim][j] = v;
-        else
-            sdth[row][dim][j] = v;
-    }
-    const int bl = hl < 3 ? dv.pmeBase[3 * i + hl] : 0;
-    const int b0 = __shfl_sync(mask, bl, 0, L), b1 = __shfl_sync(mask, bl, 1, L), b2 = __shfl_sync(mask, bl, 2, L);
-    __syncwarp(mask);
-    const int K0 = S.K[0], K1 = S.K[1], K2 = S.K[2];
-    const size_t plane = (size_t) K1 * K2;
-    float f0 = 0.f, f1 = 0.f, f2 = 0.f;
-    for (int c = hl; c < P * P; c += L) {
-        const int j2 = c / P, j3 = c % P;
-        const float* col = gpot + (size_t) wrapIndex(b1 - j2, K1) * K2 + wrapIndex(b2 - j3, K2);
-        float St = 0.f, Su = 0.f;
-#pragma unroll
-        for (int j1 = 0; j1 < P; j1++) {
-            const float ph = __ldcg(col + (size_t) wrapIndex(b0 - j1, K0) * plane);
-            St += sth[row][0][j1] * ph;
-            Su += sdth[row][0][j1] * ph;
-        }
-        const float t2 = sth[row][1][j2], u2 = sdth[row][1][j2];
-        const float t3 = sth[row][2][j3], u3 = sdth[row][2][j3];
-        f0 += Su * t2 * t3;
-        f1 += St * u2 * t3;
-        f2 += St * t2 * u3;
-    }
-    double F[3] = {(double) f0, (double) f1, (double) f2};
-#pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            F[k] += __shfl_xor_sync(mask, F[k], o, L);
-    double share = 0.0;
-    if (hl < 3) {
-        const int k = hl;
-        const double E = -(S.K[0] * S.recip[3 * k] * F[0] + S.K[1] * S.recip[3 * k + 1] * F[1] +
-                           S.K[2] * S.recip[3 * k + 2] * F[2]);
-        if (CGA) {
-            const double Tp = eI + E + cs * pI;
-            const double apk = (alI > 0) ? pI / alI - Tp : 0.0;
-            dv.Ap[3 * i + k] = apk;
-            share = pI * apk;
-        } else {
-            dv.Erec[3 * i + k] = E;
-        }
-    }
-    __syncwarp(mask);
-    return share;
+// A load that leaves no line behind in L1 (the pair records, read once per pass).
+__device__ __forceinline__ float4 loadStreaming(const float4* p) {
+    float4 v;
+    asm("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 loadStreaming(const float2* p) {
+    float2 v;
+    asm("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
 }
 
-// Direct-space field of the direction p (mixed pair records) at slots g0, g0 + gstride, ...: GS lanes per slot,
-// E_i = sum_j -p_j G1 + (p_j . x) x G2 (core/pgm_core.cpp:274-284), products in float, sums across lanes in
-// double, written to Epair (caller order).
-template <int GS, bool WITHQ>
-__device__ __forceinline__ void pcgPairField(const Dev& dv, int g0, int gstride) {
-    const int lane = threadIdx.x % GS;
-    const unsigned gm = groupMask<GS>();
+// Direct-space field of the dipoles dS (mixed pair records) at slots s0 .. s1 - 1, a warp per slot: E_i = sum_j -p_j G1 +
+// (p_j . x) x G2 (core/pgm_core.cpp:274-284), products in float, sums across lanes in double, written to E (slot order).
+__device__ __forceinline__ void pcgPairField(const Dev& dv, double* E, int s0, int s1) {
+    const int lane = threadIdx.x & 31;
     const float4* dS = (const float4*) dv.dS;
-    for (int slot = g0; slot < dv.nAtoms; slot += gstride) {
+    for (int slot = s0 + (threadIdx.x >> 5); slot < s1; slot += PCG_THREADS / 32) {
         const float4* arow = (const float4*) dv.pairA + (size_t) slot * dv.cap;
         const float2* brow = (const float2*) dv.pairB + (size_t) slot * dv.cap;
         const int cnt = dv.listCount[slot];
         float a0 = 0.f, a1 = 0.f, a2 = 0.f;
 #pragma unroll 4
-        for (int t = lane; t < cnt; t += GS) {
-            const float4 xg = arow[t];
-            const float2 gb = brow[t];
-            const float4 dj = __ldcg(dS + realAsSlot(gb.y));   // (written by other blocks in this launch)
-            float c = (dj.x * xg.x + dj.y * xg.y + dj.z * xg.z) * gb.x;
-            if (WITHQ)
-                c += dj.w * xg.w;
+        for (int t = lane; t < cnt; t += 32) {
+            const float4 xg = loadStreaming(arow + t);
+            const float2 gb = loadStreaming(brow + t);
+            const float4 dj = dS[realAsSlot(gb.y)];
+            const float c = (dj.x * xg.x + dj.y * xg.y + dj.z * xg.z) * gb.x;
             a0 += c * xg.x - dj.x * xg.w;
             a1 += c * xg.y - dj.y * xg.w;
             a2 += c * xg.z - dj.z * xg.w;
         }
         double E0 = a0, E1 = a1, E2 = a2;
 #pragma unroll
-        for (int o = GS / 2; o > 0; o >>= 1) {
-            E0 += __shfl_xor_sync(gm, E0, o, GS);
-            E1 += __shfl_xor_sync(gm, E1, o, GS);
-            E2 += __shfl_xor_sync(gm, E2, o, GS);
+        for (int o = 16; o > 0; o >>= 1) {
+            E0 += __shfl_xor_sync(0xffffffffu, E0, o);
+            E1 += __shfl_xor_sync(0xffffffffu, E1, o);
+            E2 += __shfl_xor_sync(0xffffffffu, E2, o);
         }
-        if (lane == 0) {
-            const int i = dv.slotAtom[slot];
-            dv.Epair[3 * i] = E0;
-            dv.Epair[3 * i + 1] = E1;
-            dv.Epair[3 * i + 2] = E2;
-        }
+        if (lane < 3)
+            E[3 * (size_t) slot + lane] = lane == 0 ? E0 : lane == 1 ? E1 : E2;
     }
 }
 
-// Block-wide fixed-order sum (or max where the bit of maxMask is set) of NV values per block over the nb
-// blocks' shares part[b * 4 + k]; every block obtains the same totals.
-template <int NV>
-__device__ __forceinline__ void pcgTotals(const double* part, int nb, unsigned maxMask, double* tot) {
-    double v[NV];
+// Sums over a warp (or the largest, where the bit of maxMask is set), in every lane.
+template <int NV> __device__ __forceinline__ void pcgWarpSums(double* v, unsigned maxMask) {
 #pragma unroll
-    for (int k = 0; k < NV; k++)
-        v[k] = 0.0;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x)
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
         for (int k = 0; k < NV; k++) {
-            const double x = __ldcg(part + (size_t) b * 4 + k);
-            v[k] = ((maxMask >> k) & 1u) ? fmax(v[k], x) : v[k] + x;
+            const double y = __shfl_xor_sync(0xffffffffu, v[k], o);
+            v[k] = ((maxMask >> k) & 1u) ? fmax(v[k], y) : v[k] + y;
         }
-    blockReduce<NV>(v, maxMask);
-    __shared__ double out[NV];
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < NV; k++)
-            out[k] = v[k];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NV; k++)
-        tot[k] = out[k];
-    __syncthreads();
 }
 
-// KC > 0: the grid is KC^3 (compile-time line transforms); 0: any grid the plane blocks handle.
-// PASS 0: the CG loop.  PASS 1 / 2: ONE field pass of the same machinery -- the field at every atom of the dipoles
-// vec (2: and the charges), E_pair and E_rec written per atom -- for the passes around the loop.
-template <int P, int GS, int KC, int PASS>
-__global__ void __launch_bounds__(PCG_THREADS, PCG_BLOCKS_PER_SM) k_cg_persistent(Dev dv, int nyc, const double* vec) {
+// The block's share of NV values into part[k * nb + x] (thread 0), in a fixed order; one block barrier.
+template <int NV>
+__device__ __forceinline__ void pcgShare(double* v, unsigned maxMask, double* part, int nb) {
+    __shared__ double red[NV][PCG_THREADS / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    pcgWarpSums<NV>(v, maxMask);
+    if (lane < NV)
+        red[lane][wid] = NV == 1 || lane == 0 ? v[0] : lane == 1 ? v[NV > 1 ? 1 : 0] : v[NV > 2 ? 2 : 0];
+    __syncthreads();
+    if (wid == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; k++)
+            v[k] = red[k][lane];
+        pcgWarpSums<NV>(v, maxMask);
+        if (lane == 0)
+#pragma unroll
+            for (int k = 0; k < NV; k++)
+                part[(size_t) k * nb + blockIdx.x] = v[k];
+    }
+}
+
+// The blocks' shares part[k * nb + b] of NV values, summed (or the largest) in a fixed order by every warp for itself:
+// after a barrier of the blocks, without one of the block's own.
+template <int NV>
+__device__ __forceinline__ void pcgTotals(const double* part, int nb, unsigned maxMask, double* tot) {
+    const int lane = threadIdx.x & 31;
+    double x[NV][PCG_MAX_BLOCKS / 32];
+#pragma unroll
+    for (int k = 0; k < NV; k++)
+#pragma unroll
+        for (int m = 0; m < PCG_MAX_BLOCKS / 32; m++)
+            x[k][m] = lane + 32 * m < nb ? part[(size_t) k * nb + lane + 32 * m] : 0.0;
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        tot[k] = x[k][0];
+#pragma unroll
+        for (int m = 1; m < PCG_MAX_BLOCKS / 32; m++)
+            tot[k] = ((maxMask >> k) & 1u) ? fmax(tot[k], x[k][m]) : tot[k] + x[k][m];
+    }
+    pcgWarpSums<NV>(tot, maxMask);
+}
+
+// KC > 0: the grid is KC^3 (compile-time line transforms); 0: any grid the plane blocks handle.  The right-hand side is
+// E_perm = E_pair + E_rec + self field of the permanent dipoles (written to b), or, with the control's customRhs, b.
+// planeSlots: the rows of the pair pass that a plane block's transforms are worth.
+template <int P, int KC>
+__global__ void __launch_bounds__(PCG_THREADS, 1) k_cg_persistent(Dev dv, int planeSlots) {
     typedef cufftComplex C;
+    constexpr int SL = PCG_SLOT_LANES;
     const SysDev& S = dv.sys[0];
     double* sc = dv.scal;
-    if (PASS == 0 && sc[SC_DONE] != 0.0)
-        return;   // converged at the initial guess (every block alike)
     const int n = dv.nAtoms, nb = gridDim.x, tid = threadIdx.x, nT = blockDim.x;
     const int K0 = KC > 0 ? KC : S.K[0], K1 = KC > 0 ? KC : S.K[1], K2 = KC > 0 ? KC : S.K[2];
     const int x = blockIdx.x;
     const bool planeBlock = x < K0;
     unsigned* const gbar = dv.pcgBar;        // every block
     unsigned* const pbar = dv.pcgBar + 1;    // the plane blocks
+    const int per = (n + nb - 1) / nb, s0 = min(n, x * per), ns = min(n, s0 + per) - s0;
     extern __shared__ __align__(16) unsigned char smraw[];
     C* W0 = (C*) smraw;
     C* W1 = W0 + FFT_MAXK;
     C* W2 = W1 + FFT_MAXK;
     C* const b0 = W2 + FFT_MAXK;
     C* const b1 = b0 + dv.fftgBuf;
+    double* const sx = (double*) (b1 + dv.fftgBuf);   // the slots' x, r, p, A p (3 per slot), alpha
+    double* const sr = sx + 3 * per;
+    double* const sp = sr + 3 * per;
+    double* const sAp = sp + 3 * per;
+    double* const sal = sAp + 3 * per;
+    float* const spl = (float*) (sal + per);
+    int* const satom = (int*) (spl + PCG_SPL * per);
+    int* const sbase = satom + per;
     const C* tw = (const C*) dv.twiddle;
     if (planeBlock) {
         for (int m = tid; m < K0; m += nT)
@@ -270,180 +196,233 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_BLOCKS_PER_SM) k_cg_persisten
         for (int m = tid; m < K2; m += nT)
             W2[m] = tw[S.twOff[2] + m];
     }
+    for (int s = tid; s < ns; s += nT) {
+        const int i = dv.slotAtom[s0 + s];
+        satom[s] = i;
+        sal[s] = dv.alpha[i];
+        for (int k = 0; k < 3; k++)
+            sbase[3 * s + k] = dv.pmeBase[3 * i + k];
+    }
+    for (int t = tid; t < ns * 6 * P; t += nT) {   // (the evaluation's coefficients, rows of MAXP)
+        const int s = t / (6 * P), k = t - s * 6 * P;
+        spl[s * PCG_SPL + k] = ((const float*) dv.spl)[(size_t) (s0 + s) * 9 * MAXP + (k / P) * MAXP + k % P];
+    }
+    __syncthreads();
     const PlaneFft<float, KC> fft(K0, K1, K2, b0, b1, W0, W1, W2);
     const int nline = fft.nline, l0 = x * fft.lpb, nl = min(nline, l0 + fft.lpb) - l0;
     C* const spec = (C*) dv.spec + S.specOff;
-    double* const part = dv.pcgPartial;
-    // the slot-group phases (spread, gather): the groups' shared spline rows, the fixed-point charge grid and the
-    // float potential grid
-    constexpr int SL = PCG_SLOT_LANES;
-    __shared__ float psth[PCG_THREADS / SL][3][P], psdth[PCG_THREADS / SL][3][P];
-    // the slot-group phases: SL lanes per slot
-    const int hrow = tid / SL, hl = tid % SL, nhalves = nT / SL;
-    const unsigned hmask = ((1u << SL) - 1u) << (tid & 31 & ~(SL - 1));
+    const float* const infl = (const float*) dv.infl + S.specOff;
     long long* const gfix = dv.gridFix + S.gridOff;
     float* const gpot = (float*) dv.grid + S.gridOff;
-    (void) nyc;
+    double* const Eslot = dv.Fpair;          // (the pair field in slot order; the final pass writes Fpair later)
+    double* const partA = dv.pcgPartial;     // shares of three sums, and of the two around the next spread
+    double* const partB = partA + 3 * nb;
+    const int hrow = tid / SL, hl = tid % SL, rows = nT / SL;
+    const unsigned hmask = groupMask<SL>();
+    // the pair pass's rows: q for a plane block, planeSlots more for the others
+    const int q = max(0, (n - (nb - K0) * planeSlots + nb - 1) / nb);
+    const int rest = (max(0, n - K0 * q) + nb - K0 - 1) / (nb - K0);
+    const int g0 = min(n, planeBlock ? x * q : K0 * q + (x - K0) * rest), g1 = min(n, g0 + (planeBlock ? q : rest));
+    const size_t plane = (size_t) K1 * K2;
     const double cs = 4.0 * S.beta * S.beta * S.beta / (3.0 * SQRT_PI);
-    // the block's chunk of slots for the per-atom phases
-    const int per = (n + nb - 1) / nb, s0 = x * per, s1 = min(n, s0 + per);
-    double rz = sc[SC_RZ], beta = sc[SC_BETA], it = sc[SC_IT];
-    const double norm = sc[SC_NORM];
-    for (;;) {
-        // ---- S: SL lanes per slot: direction p = z + beta p (or the pass's sources), the float copy for the
-        // pair pass, the PME weights (q, e_a = K_a p . recip[:, a]) and the spread
-        for (int s = s0 + hrow; s < s1; s += nhalves) {
-            const int i = dv.slotAtom[s];
-            SpreadPre<P, SL> pre;
-            pre.load(dv, s, i, hl);
-            double dl = 0.0;
-            if (hl < 3) {
-                if (PASS == 0) {
-                    dl = dv.z[3 * i + hl] + beta * dv.p[3 * i + hl];
-                    dv.p[3 * i + hl] = dl;
-                } else {
-                    dl = vec[3 * i + hl];
-                }
-            }
-            const double d0 = __shfl_sync(hmask, dl, 0, SL), d1 = __shfl_sync(hmask, dl, 1, SL),
-                         d2 = __shfl_sync(hmask, dl, 2, SL);
-            const float qf = PASS == 2 ? (float) dv.q[i] : 0.f;
+    const bool custom = dv.ctl->customRhs != 0;
+    const int guess = dv.ctl->guess;
+
+    // S: the vector v (3 per slot) as sources
+    auto spread = [&](const double* v) {
+        for (int s = hrow; s < ns; s += rows) {
+            const double d0 = v[3 * s], d1 = v[3 * s + 1], d2 = v[3 * s + 2];
             if (hl == 0)
-                ((float4*) dv.dS)[s] = make_float4((float) d0, (float) d1, (float) d2, qf);
-            const float4 w = make_float4(qf, (float) (S.K[0] * (d0 * S.recip[0] + d1 * S.recip[3] + d2 * S.recip[6])),
-                                         (float) (S.K[1] * (d0 * S.recip[1] + d1 * S.recip[4] + d2 * S.recip[7])),
-                                         (float) (S.K[2] * (d0 * S.recip[2] + d1 * S.recip[5] + d2 * S.recip[8])));
-            pcgSpreadHalf<P, SL>(dv, S, gfix, w, pre, psth, psdth, hrow, hl, hmask);
+                ((float4*) dv.dS)[s0 + s] = make_float4((float) d0, (float) d1, (float) d2, 0.f);
+            const float e0 = (float) (S.K[0] * (d0 * S.recip[0] + d1 * S.recip[3] + d2 * S.recip[6])),
+                        e1 = (float) (S.K[1] * (d0 * S.recip[1] + d1 * S.recip[4] + d2 * S.recip[7])),
+                        e2 = (float) (S.K[2] * (d0 * S.recip[2] + d1 * S.recip[5] + d2 * S.recip[8]));
+            const float* th = spl + s * PCG_SPL;
+            const int bs0 = sbase[3 * s], bs1 = sbase[3 * s + 1], bs2 = sbase[3 * s + 2];
+            int off[P];
+#pragma unroll
+            for (int j1 = 0; j1 < P; j1++)
+                off[j1] = wrapIndex(bs0 - j1, K0) * (int) plane;
+            for (int c = hl; c < P * P; c += SL) {
+                const int j2 = c / P, j3 = c % P;
+                const float t2 = th[P + j2], u2 = th[4 * P + j2], t3 = th[2 * P + j3], u3 = th[5 * P + j3];
+                const float c23 = t2 * t3;
+                const float a = e1 * u2 * t3 + e2 * t2 * u3, b = e0 * c23;
+                long long* col = gfix + wrapIndex(bs1 - j2, K1) * K2 + wrapIndex(bs2 - j3, K2);
+#pragma unroll
+                for (int j1 = 0; j1 < P; j1++)
+                    gridFixAdd(col + off[j1], a * th[j1] + b * th[3 * P + j1]);
+            }
         }
-        if (!fftgBarrier(gbar, (unsigned) nb, dv.flags))
-            return;
-        // ---- F: the plane blocks' reciprocal part, the other blocks' direct part
+    };
+    // F and G: T v = pair + reciprocal + self field; the rows of A v = v / alpha - T v (0 where not polarizable) in
+    // sAp.  The caller's barrier came after the spread; false: a barrier gave up.
+    auto apply = [&](const double* v) -> bool {
         if (planeBlock) {
-            // plane x from the fixed-point grid (cleared for the next spread), its share of the x-lines with the
-            // influence product, and back into the potential grid
-            long long* const fxx = gfix + (size_t) x * K1 * K2;
+            long long* const fxx = gfix + (size_t) x * plane;
             fft.forward(
                 [&](int e) {
-                    const long long v = __ldcg(fxx + e);
+                    const long long w = __ldcg(fxx + e);
                     __stcg(fxx + e, 0ll);
-                    return (float) ((double) v * (1.0 / 4294967296.0));
+                    return gridFixValue(w);
                 },
                 spec + (size_t) x * nline);
             if (!fftgBarrier(pbar, (unsigned) K0, dv.flags))
-                return;
-            const float* infl = (const float*) dv.infl + S.specOff;
-            fft.lines(spec, l0, nl, [&](int m1, int l, C v) {
+                return false;
+            fft.lines(spec, l0, nl, [&](int m1, int l, C w) {
                 const float gk = infl[(size_t) m1 * nline + l];
-                v.x *= gk;
-                v.y *= gk;
-                return v;
+                w.x *= gk;
+                w.y *= gk;
+                return w;
             });
             if (!fftgBarrier(pbar, (unsigned) K0, dv.flags))
+                return false;
+            float* const gx = gpot + (size_t) x * plane;
+            fft.inverse(spec + (size_t) x * nline, [&](int e, float w) { gx[e] = w; });
+        }
+        pcgPairField(dv, Eslot, g0, g1);
+        if (!fftgBarrier(gbar, (unsigned) nb, dv.flags))
+            return false;
+        for (int s = hrow; s < ns; s += rows) {
+            double eP = 0.0;
+            if (hl < 3)
+                eP = Eslot[3 * (size_t) (s0 + s) + hl];
+            const float* th = spl + s * PCG_SPL;
+            const int bs0 = sbase[3 * s], bs1 = sbase[3 * s + 1], bs2 = sbase[3 * s + 2];
+            int off[P];
+#pragma unroll
+            for (int j1 = 0; j1 < P; j1++)
+                off[j1] = wrapIndex(bs0 - j1, K0) * (int) plane;
+            float f0 = 0.f, f1 = 0.f, f2 = 0.f;
+#pragma unroll
+            for (int c = hl; c < P * P; c += SL) {
+                const int j2 = c / P, j3 = c % P;
+                const float* col = gpot + wrapIndex(bs1 - j2, K1) * K2 + wrapIndex(bs2 - j3, K2);
+                float St = 0.f, Su = 0.f;
+#pragma unroll
+                for (int j1 = 0; j1 < P; j1++) {
+                    const float ph = col[off[j1]];
+                    St += th[j1] * ph;
+                    Su += th[3 * P + j1] * ph;
+                }
+                const float t2 = th[P + j2], u2 = th[4 * P + j2], t3 = th[2 * P + j3], u3 = th[5 * P + j3];
+                f0 += Su * t2 * t3;
+                f1 += St * u2 * t3;
+                f2 += St * t2 * u3;
+            }
+            double F0 = f0, F1 = f1, F2 = f2;
+#pragma unroll
+            for (int o = SL / 2; o > 0; o >>= 1) {
+                F0 += __shfl_xor_sync(hmask, F0, o, SL);
+                F1 += __shfl_xor_sync(hmask, F1, o, SL);
+                F2 += __shfl_xor_sync(hmask, F2, o, SL);
+            }
+            if (hl < 3) {
+                const double E = -(S.K[0] * S.recip[3 * hl] * F0 + S.K[1] * S.recip[3 * hl + 1] * F1 +
+                                   S.K[2] * S.recip[3 * hl + 2] * F2);
+                const double al = sal[s], vk = v[3 * s + hl], T = eP + E + cs * vk;
+                sAp[3 * s + hl] = (al > 0) ? vk / al - T : 0.0;
+            }
+        }
+        __syncthreads();
+        return true;
+    };
+
+    // b, x0 and the share of sum |alpha b|
+    {
+        const size_t hs = (size_t) 3 * dv.numGlobal;
+        double v[1] = {0.0};
+        for (int t = tid; t < 3 * ns; t += nT) {
+            const int s = t / 3, k = t - 3 * s, i = satom[s];
+            const int gi = dv.globalIndex ? dv.globalIndex[i] : i;
+            const double al = sal[s];
+            const double bk = custom ? dv.b[3 * i + k] : dv.Epair[3 * i + k] + dv.Erec[3 * i + k] + cs * dv.perm[3 * i + k];
+            if (!custom)
+                dv.b[3 * i + k] = bk;
+            v[0] += fabs(al * bk);
+            const double x0 = guess == 0 ? al * bk : historyGuess(dv, guess, (size_t) 3 * gi + k, hs);
+            sx[t] = (guess >= 2 && !(al > 0)) ? 0.0 : x0;
+            sr[t] = bk;
+        }
+        pcgShare<1>(v, 0u, partA, nb);   // (its barrier also publishes sx)
+    }
+    // The first round forms r = b - A x0 (from the zero guess r = b, without a pass), every later one is an iteration.
+    // (One call of spread and of apply in the code: a second would put what they capture into local memory.)
+    double norm = 0.0, rz = 0.0, err = 0.0, it = 0.0;
+    for (bool first = true;; first = false) {
+        if (!first || guess != 1) {
+            const double* const src = first ? sx : sp;
+            spread(src);
+            if (!fftgBarrier(gbar, (unsigned) nb, dv.flags))
                 return;
-            float* const gx = gpot + (size_t) x * K1 * K2;   // plane x of the potential
-            fft.inverse(spec + (size_t) x * nline, [&](int e, float v) { gx[e] = v; });
+            if (!first) {   // r.z, and the convergence test on max |z|: they went around with this barrier
+                double tot[2];
+                if (it == 0.0) {
+                    pcgTotals<1>(partA, nb, 0u, tot);
+                    norm = tot[0] / (3.0 * n) + 1e-300;
+                }
+                pcgTotals<2>(partB, nb, 2u, tot);
+                rz = tot[0];
+                err = tot[1] / norm;
+                if (!(err > dv.tol && it < dv.maxIter)) {
+                    if (planeBlock)   // the dropped direction's spread
+                        for (int e = tid; e < (int) plane; e += nT)
+                            __stcg(gfix + (size_t) x * plane + e, 0ll);
+                    break;
+                }
+            }
+            if (!apply(src))
+                return;
+        }
+        double w[2] = {0.0, 0.0};
+        if (first) {   // r = b - A x0 (rows of polarizable atoms); the first direction is z
+            for (int t = tid; t < 3 * ns; t += nT) {
+                const double al = sal[t / 3];
+                const double rk = (al > 0) ? (guess != 1 ? sr[t] - sAp[t] : sr[t]) : 0.0, zk = al * rk;
+                sr[t] = rk;
+                sp[t] = zk;
+                w[0] += rk * zk;
+                w[1] = fmax(w[1], fabs(zk));
+            }
         } else {
-            const int groups = nT / GS;
-            pcgPairField<GS, PASS == 2>(dv, (x - K0) * groups + tid / GS, (nb - K0) * groups);
-        }
-        if (!fftgBarrier(gbar, (unsigned) nb, dv.flags))
-            return;
-        // ---- G: E_rec at the chunk's atoms (a field pass), or the rows of A p and the block's share of p . A p
-        if (PASS != 0) {   // one field pass: E_pair and E_rec written
-            for (int s = s0 + hrow; s < s1; s += nhalves)
-                pcgGatherHalf<P, false, SL>(dv, S, gpot, s, psth, psdth, hrow, hl, hmask, cs);
-            return;
-        }
-        {
-            double v[1] = {0.0};
-            for (int s = s0 + hrow; s < s1; s += nhalves)
-                v[0] += pcgGatherHalf<P, true, SL>(dv, S, gpot, s, psth, psdth, hrow, hl, hmask, cs);
-            blockReduce<1>(v, 0u);
-            if (tid == 0)
-                part[(size_t) x * 4] = v[0];
-        }
-        if (!fftgBarrier(gbar, (unsigned) nb, dv.flags))
-            return;
-        // ---- U: alph, x, r, z; shares of z'.(r' - r), r'.z', max|z'|
-        {
-            // the first slot's p, x, r, A p and alpha are loaded before the total of p . A p is formed
-            const int sF = s0 + tid;
-            const bool hasF = sF < s1;
-            const int iF = hasF ? dv.slotAtom[sF] : 0;
-            double pF[3] = {0, 0, 0}, xF[3] = {0, 0, 0}, rF[3] = {0, 0, 0}, aF[3] = {0, 0, 0}, alF = 0.0;
-            if (hasF) {
-                alF = dv.alpha[iF];
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    pF[k] = dv.p[3 * iF + k];
-                    xF[k] = dv.x[3 * iF + k];
-                    rF[k] = dv.r[3 * iF + k];
-                    aF[k] = dv.Ap[3 * iF + k];
-                }
-            }
-            double pap[1];
-            pcgTotals<1>(part, nb, 0u, pap);
-            const double alph = rz / fmax(pap[0], 1e-300);
             double v[3] = {0.0, 0.0, 0.0};
-            auto update = [&](int i, double al, const double* pk, const double* xk, const double* rk, const double* ak) {
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    dv.x[3 * i + k] = xk[k] + alph * pk[k];
-                    const double rold = rk[k];
-                    const double rn = rold - alph * ak[k];
-                    const double zn = al * rn;
-                    dv.r[3 * i + k] = rn;
-                    dv.z[3 * i + k] = zn;
-                    v[0] += zn * (rn - rold);
-                    v[1] += rn * zn;
-                    v[2] = fmax(v[2], fabs(zn));
-                }
-            };
-            if (hasF)
-                update(iF, alF, pF, xF, rF, aF);
-            for (int s = sF + nT; s < s1; s += nT) {
-                const int i = dv.slotAtom[s];
-                double pk[3], xk[3], rk[3], ak[3];
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    pk[k] = dv.p[3 * i + k];
-                    xk[k] = dv.x[3 * i + k];
-                    rk[k] = dv.r[3 * i + k];
-                    ak[k] = dv.Ap[3 * i + k];
-                }
-                update(i, dv.alpha[i], pk, xk, rk, ak);
+            for (int t = tid; t < 3 * ns; t += nT) {
+                const double al = sal[t / 3], a = sAp[t], za = al * a;
+                v[0] += sp[t] * a;
+                v[1] += sr[t] * za;
+                v[2] += a * za;
             }
-            blockReduce<3>(v, 4u);
-            if (tid == 0) {
-                if (x == 0)
-                    sc[SC_ALPH] = alph;
-                part[(size_t) nb * 4 + (size_t) x * 4] = v[0];
-                part[(size_t) nb * 4 + (size_t) x * 4 + 1] = v[1];
-                part[(size_t) nb * 4 + (size_t) x * 4 + 2] = v[2];
+            pcgShare<3>(v, 0u, partA, nb);
+            if (!fftgBarrier(gbar, (unsigned) nb, dv.flags))
+                return;
+            double tot[3];
+            pcgTotals<3>(partA, nb, 0u, tot);
+            const double alph = rz / fmax(tot[0], 1e-300);
+            const double beta = -alph * (tot[1] - alph * tot[2]) / fmax(rz, 1e-300);
+            it += 1.0;
+            for (int t = tid; t < 3 * ns; t += nT) {
+                const double pk = sp[t], rn = sr[t] - alph * sAp[t], zn = sal[t / 3] * rn;
+                sx[t] += alph * pk;
+                sr[t] = rn;
+                sp[t] = zn + beta * pk;
+                w[0] += rn * zn;
+                w[1] = fmax(w[1], fabs(zn));
             }
         }
-        if (!fftgBarrier(gbar, (unsigned) nb, dv.flags))
-            return;
-        // ---- C: the same decision in every block
-        double tot[3];
-        pcgTotals<3>(part + (size_t) nb * 4, nb, 4u, tot);
-        beta = tot[0] / fmax(rz, 1e-300);
-        rz = tot[1];
-        const double err = tot[2] / norm;
-        it += 1.0;
-        const bool more = err > dv.tol && it < dv.maxIter;
-        if (x == 0 && tid == 0) {
-            sc[SC_BETA] = beta;
-            sc[SC_RZ] = rz;
-            sc[SC_ERR] = err;
-            sc[SC_IT] = it;
-            if (!more) {
-                sc[SC_DONE] = 1.0;
-                atomicAdd(&dv.flags[2], 1);
-            }
-        }
-        if (!more)
-            return;
+        pcgShare<2>(w, 2u, partB, nb);
+    }
+    for (int t = tid; t < 3 * ns; t += nT) {
+        const int i = satom[t / 3], k = t % 3;
+        dv.x[3 * i + k] = sx[t];
+        dv.r[3 * i + k] = sr[t];
+    }
+    if (x == 0 && tid == 0) {
+        sc[SC_NORM] = norm;
+        sc[SC_RZ] = rz;
+        sc[SC_ERR] = err;
+        sc[SC_IT] = it;
+        sc[SC_DONE] = 1.0;
+        atomicAdd(&dv.flags[2], 1);
     }
 }
 

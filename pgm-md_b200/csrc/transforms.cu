@@ -1,6 +1,6 @@
 #include "transforms.cuh"
 
-#include "persistent.cuh"
+#include "gridfft.cuh"
 
 namespace pgmb200 {
 
@@ -15,17 +15,5 @@ template <typename R> GridKernel gridKernel(int kc, bool energy) {
 }
 template GridKernel gridKernel<float>(int, bool);
 template GridKernel gridKernel<double>(int, bool);
-
-template <int GS, int KC> static PcgKernel pcgPass(int pass) {
-    return pass == 0 ? k_cg_persistent<6, GS, KC, 0> : pass == 1 ? k_cg_persistent<6, GS, KC, 1> : k_cg_persistent<6, GS, KC, 2>;
-}
-
-PcgKernel pcgKernel(int lanes, int kc, int pass) {
-    if (lanes >= 32)
-        return kc == 48 ? pcgPass<32, 48>(pass) : pcgPass<32, 0>(pass);
-    if (lanes >= 16)
-        return kc == 48 ? pcgPass<16, 48>(pass) : pcgPass<16, 0>(pass);
-    return kc == 48 ? pcgPass<8, 48>(pass) : pcgPass<8, 0>(pass);
-}
 
 }  // namespace pgmb200

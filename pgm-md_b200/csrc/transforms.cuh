@@ -10,9 +10,8 @@ namespace pgmb200 {
 typedef void (*GridKernel)(Dev, int);
 template <typename R> GridKernel gridKernel(int kc, bool energy);
 
-// The persistent CG kernel for the pair lanes (8, 16 or 32; 4 runs as 8) and the grid's compile-time size (48, or 0:
-// any).  pass 0: the CG loop; 1 / 2: one field pass of dipoles (and charges).
-typedef void (*PcgKernel)(Dev, int, const double*);
-PcgKernel pcgKernel(int lanes, int kc, int pass);
+// The persistent CG kernel, compiled for the cubic grids of pcgSizes; any other grid (kc = 0) takes the general one.
+typedef void (*PcgKernel)(Dev, int);
+PcgKernel pcgKernel(int kc);
 
 }  // namespace pgmb200
