@@ -65,7 +65,9 @@ __global__ void k_fm_dp(Dev dv, const double* w, double* dp) {
 //                   - (d_j.x) x G3 (x.dx)
 //   D gR_i  = sum_j D U_a (-2 R_i a^3),  D U_a the pair energy with G_n -> H_n differentiated,
 // x = r_i - r_j, dx = dr_i - dr_j, d the final total dipoles.  Double precision, GS lanes per atom.
-template <int GS>
+// STORED (an FP64 engine): G_1, G_2, G_3 from the evaluation's pair records; a mixed engine's are in float, so it forms
+// them again in double.
+template <int GS, bool STORED>
 __global__ void __launch_bounds__(256) k_pair_tangent(Dev dv, const double* dr, const double* dd, double* Dphi,
                                                       double* DE, double* DgR) {
     const int slot = (blockIdx.x * blockDim.x + threadIdx.x) / GS, lane = threadIdx.x % GS;
@@ -94,7 +96,14 @@ __global__ void __launch_bounds__(256) k_pair_tangent(Dev dv, const double* dr, 
         const double Rj = dv.radS[js];
         const double a = 1.0 / sqrt(2.0 * (Ri * Ri + Rj * Rj));
         double G[4];
-        pairKernels<double, 4>(a, S.beta, r, G);
+        if (STORED) {
+            const double2 gb = ((const double2*) dv.pairB)[(size_t) slot * dv.cap + t];
+            G[1] = gb.x;
+            G[2] = gb.y;
+            G[3] = ((const double2*) dv.pairC)[(size_t) slot * dv.cap + t].y;
+        } else {
+            pairKernels<double, 4>(a, S.beta, r, G);
+        }
         const double qj = pwj.w;
         const double dj[3] = {dv.dtot[3 * j], dv.dtot[3 * j + 1], dv.dtot[3 * j + 2]};
         const double ddj[3] = {dd[3 * j], dd[3 * j + 1], dd[3 * j + 2]};
