@@ -289,70 +289,6 @@ __device__ __forceinline__ void pairKernels(R a, R beta, R r, R* G) {
         G[k] -= B[k];
 }
 
-// 1 / sqrt(v) to about half an ulp: the hardware's approximation and one Newton step.
-__device__ __forceinline__ float rsqrtNewton(float v) {
-    const float y = rsqrtf(v), e = fmaf(-v * y, y, 1.0f);
-    return fmaf(0.5f * y, e, y);
-}
-
-// B_0..B_3 of erfc(s r)/r by the all-positive recursion (core/pgm_math.h:63-75) in float, with ONE exponential:
-// erfc(x) = exp(-x^2) F / (1 + 2x), F = (1 + 2x) exp(x^2) erfc(x) a polynomial in (x - 2)/(x + 2) (Shepherd and Laframboise,
-// Math. Comp. 36 (1981) 249, the form; the coefficients are a Chebyshev fit of degree 11 on 0 <= x < inf, 1.1e-8 off
-// before rounding).  The rounding of x^2 is carried into the exponential, so erfc errs by 3.6e-7 at most and 7.6e-8 RMS
-// (relative, 0 <= x <= 6).
-__device__ __forceinline__ void erfcRecord(float s, float r, float ir, float ir2, float* B) {
-    const float x = s * r, x2 = x * x, lo = fmaf(x, x, -x2);
-    float E = expf(-x2);
-    E = fmaf(-E, lo, E);
-    const float t1 = fmaf(2.0f, x, 1.0f), t2 = x + 2.0f, t12 = t1 * t2, w0 = __fdividef(1.0f, t12);
-    const float w = fmaf(w0, fmaf(-t12, w0, 1.0f), w0);
-    const float q = (x - 2.0f) * (t1 * w);
-    float F = 6.336945807561278e-05f;
-    F = fmaf(F, q, 0.0001608035818208009f);
-    F = fmaf(F, q, -0.0003579204494599253f);
-    F = fmaf(F, q, -0.0013957069022580981f);
-    F = fmaf(F, q, 0.0012174105504527688f);
-    F = fmaf(F, q, 0.008689159527420998f);
-    F = fmaf(F, q, -0.008018963038921356f);
-    F = fmaf(F, q, -0.05421195924282074f);
-    F = fmaf(F, q, 0.16404946148395538f);
-    F = fmaf(F, q, -0.1660310924053192f);
-    F = fmaf(F, q, -0.0927637591958046f);
-    F = fmaf(F, q, 1.2769783735275269f);
-    B[0] = E * F * (t2 * w) * ir;
-    const float a2 = 2.0f * s * s;
-    float c = (float) (2.0 / SQRT_PI) * s * E;
-#pragma unroll
-    for (int k = 1; k < 4; k++) {
-        B[k] = fmaf((float) (2 * k - 1), B[k - 1], c) * ir2;
-        c *= a2;
-    }
-}
-
-// The pair records' G_0..G_3 from r^2 and 1/a^2 = 2 (R_i^2 + R_j^2).  Double: pairKernels.  Float: for a r >= 2 its far
-// branch with one exponential, one division and no square root per kernel set: the record pass is bound by
-// instruction issue (about 350 a pair with erfcf, the correctly rounded divisions and square roots; RECORD_US).
-// Nearer pairs keep pairKernels: a rigid molecule has the same distances in every copy, so the rounding of their
-// kernels, the largest, adds up coherently in a parameter gradient (the 64-water loss gradient's radius element moved by
-// 8e-4 with the short form there).
-__device__ __forceinline__ void recordKernels(double r2, double ia2, double beta, double* G) {
-    pairKernels<double, 4>(1.0 / sqrt(ia2), beta, sqrt(r2), G);
-}
-__device__ __forceinline__ void recordKernels(float r2, float ia2, float beta, float* G) {
-    const float ir = rsqrtNewton(r2), r0 = r2 * ir, a = rsqrtNewton(ia2);
-    const float r = fmaf(0.5f * ir, fmaf(-r0, r0, r2), r0);   // (to half an ulp: x = s r is squared into the exponent)
-    if (!(a * r >= 2.0f)) {   // (r = 0 too)
-        pairKernels<float, 4>(1.0f / sqrtf(ia2), beta, sqrtf(r2), G);
-        return;
-    }
-    float B[4];
-    erfcRecord(beta, r, ir, ir * ir, G);
-    erfcRecord(a, r, ir, ir * ir, B);
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-        G[k] -= B[k];
-}
-
 // Cardinal B-spline values M_p(fr + j), first and second derivatives on points base - j, j < p
 // (the recursion of core/pgm_core.cpp:131-150).  Unrolled to MAXP with runtime guards so that the arrays
 // stay in registers.

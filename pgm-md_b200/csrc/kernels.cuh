@@ -333,9 +333,9 @@ __device__ __forceinline__ void minImageFast(double* v, const double* H, const d
 }
 
 constexpr int LIST_THREADS = 256;
-constexpr int LIST_ROUND = 1024;  // candidates of a round: 32 chunks of 32
-constexpr int LIST_ATOMS = 32;    // atoms of the cell taken at a time
+constexpr int LIST_CHUNK = 1024;  // candidates staged in shared memory at a time
 constexpr int MAX_RUNS = 343;     // (2m+1)^3 with m <= 3
+constexpr int NO_SHIFT = 4 | (4 << 3) | (4 << 6);   // the image code of w = 0
 
 // System of a global cell index (binary search over the systems' first cells).
 __device__ __forceinline__ int systemOfCell(const Dev& dv, int c) {
@@ -351,29 +351,23 @@ __device__ __forceinline__ int systemOfCell(const Dev& dv, int c) {
 }
 
 // One block per cell.  The neighbour cells (offsets -m..m per dimension) become at most (2m+1)^3 runs of
-// consecutive slots with one image shift each (cells along the last dimension merged).  Their atoms are the cell's
-// candidates, taken in rounds of 32 chunks of 32:
-//   1. a warp per chunk holds a candidate per lane in registers (the image's wrapped position relative to the cell's
-//      first atom, in float) and tests it against every atom of the cell, the ballots going to shared memory:
-//      - float prefilter: outside (1 + 1e-5) rl^2 is out, inside (1 - 1e-5) rl^2 with every component inside half a
-//        box edge is in (the float differences of positions within a few nm of the cell err by < 1e-6 nm^2, and
-//        a pair clearly inside the radius with its cell image inside half a box edge provably gets the same image
-//        and side from the reference's rounding);
-//      - the rest (a thin shell, or near half a box edge) takes the reference's exact test: minimum image of the
-//        original positions, r^2 < rl^2 in double without contraction (core/pgm_core.cpp:64-87), keeping the
-//        candidate only at the image that test chose, so every pair enters once;
-//   2. a warp per atom appends the round's accepted candidates to the atom's row in candidate order (deterministic;
-//      a scan over the chunks' ballots gives each its place).
-// A candidate is located, loaded and converted once for all atoms of the cell and a test costs a dozen instructions, with
-// two block barriers a round; the form before staged candidates through shared memory and gave each atom's whole row to
-// one warp, so a cell of nine atoms kept eight warps waiting for one (64 us at 8550 atoms, 440 at 98304, 4.1 ms for a
-// 1024-box batch; now LIST_US).
-__global__ void __launch_bounds__(LIST_THREADS) k_build_list(Dev dv) {
+// consecutive slots with one image shift each (cells along the last dimension merged); their atoms are
+// staged through shared memory in chunks (the image's wrapped position relative to the cell's first atom, in
+// float, and the pair entry) and every warp tests them against the cell's atoms it owns, 32 candidates at a
+// time:
+//   - float prefilter: outside (1 + 1e-5) rl^2 is out, inside (1 - 1e-5) rl^2 with every component inside half a
+//     box edge is in (the float differences of positions within a few nm of the cell err by < 1e-6 nm^2, and
+//     a pair clearly inside the radius with its cell image inside half a box edge provably gets the same image
+//     and side from the reference's rounding);
+//   - the rest (a thin shell, or near half a box edge) takes the reference's exact test: minimum image of the
+//     original positions, r^2 < rl^2 in double without contraction (core/pgm_core.cpp:64-87), keeping the
+//     candidate only at the image that test chose, so every pair enters once.
+// Accepted pairs are appended to the Verlet list (radius rl = cutoff + skin) in candidate order
+// (deterministic); k_pair_compact then takes the ones within the cutoff at every evaluation.
+__global__ void __launch_bounds__(LIST_THREADS, 4) k_build_list(Dev dv) {
     __shared__ int runSlot[MAX_RUNS], runOff[MAX_RUNS + 1], runShift[MAX_RUNS];
-    __shared__ uint32_t cEntry[LIST_ROUND];
-    __shared__ unsigned hits[LIST_ROUND / 32][LIST_ATOMS + 1];   // [chunk][atom]
-    __shared__ float4 aPos[LIST_ATOMS];
-    __shared__ int aCount[LIST_ATOMS];
+    __shared__ float4 cPos[LIST_CHUNK];
+    __shared__ uint32_t cEntry[LIST_CHUNK];
     const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     constexpr int NW = LIST_THREADS / 32;
     if (c >= dv.totalCells)
@@ -388,17 +382,18 @@ __global__ void __launch_bounds__(LIST_THREADS) k_build_list(Dev dv) {
     const int c2 = lc % n2, c1 = (lc / n2) % n1, c0 = lc / (n2 * n1);
     const int m0 = S.cellM[0], m1 = S.cellM[1], m2 = S.cellM[2];
     const int rows = (2 * m0 + 1) * (2 * m1 + 1), per = 2 * m2 + 1;
-    auto floorDiv = [](int u, int n) { return u >= 0 ? u / n : -((n - 1 - u) / n); };
     for (int row = tid; row < rows; row += LIST_THREADS) {
         const int d0 = row / (2 * m1 + 1) - m0, d1 = row % (2 * m1 + 1) - m1;
         const int u0 = c0 + d0, u1 = c1 + d1;
-        const int w0 = floorDiv(u0, n0), v0 = u0 - w0 * n0;
-        const int w1 = floorDiv(u1, n1), v1 = u1 - w1 * n1;
+        const int w0 = (int) floor((double) u0 / n0), v0 = u0 - w0 * n0;
+        const int w1 = (int) floor((double) u1 / n1), v1 = u1 - w1 * n1;
         int r = 0, d2 = -m2;
         while (d2 <= m2) {
             const int u2 = c2 + d2;
-            const int w2 = floorDiv(u2, n2), v2 = u2 - w2 * n2;
-            const int len = min(m2 - d2 + 1, n2 - v2);
+            const int w2 = (int) floor((double) u2 / n2), v2 = u2 - w2 * n2;
+            int len = 1;
+            while (d2 + len <= m2 && v2 + len < n2)
+                len++;
             const int cc = S.cellOff + (v0 * n1 + v1) * n2 + v2;
             runSlot[row * per + r] = dv.cellStart[cc];
             runOff[row * per + r] = dv.cellStart[cc + len] - dv.cellStart[cc];   // length, scanned below
@@ -433,105 +428,91 @@ __global__ void __launch_bounds__(LIST_THREADS) k_build_list(Dev dv) {
         if (lane == 0)
             runOff[nr] = carry;
     }
+    for (int ii = cb + tid; ii < ce; ii += LIST_THREADS)
+        dv.slistCount[ii] = 0;
+    __syncthreads();
+    const int total = runOff[nr];
     const double4 org = dv.posS[cb];   // the block's origin for the float positions
     const float preF = (float) (S.rl2 * (1.0 + 1e-5)), preLoF = (float) (S.rl2 * (1.0 - 1e-5));
     const float hf0 = (float) (0.5 * S.H[0] * (1.0 - 1e-5)), hf1 = (float) (0.5 * S.H[4] * (1.0 - 1e-5)),
                 hf2 = (float) (0.5 * S.H[8] * (1.0 - 1e-5));
-    for (int ab = cb; ab < ce; ab += LIST_ATOMS) {
-        const int na = min(LIST_ATOMS, ce - ab);
-        __syncthreads();   // (the runs; the rows of the atoms before these)
-        if (tid < na) {
-            const double4 p = dv.posS[ab + tid];
-            aPos[tid] = make_float4((float) (p.x - org.x), (float) (p.y - org.y), (float) (p.z - org.z), 0.0f);
-            aCount[tid] = 0;
-        }
-        const int total = runOff[nr];
-        for (int base = 0; base < total; base += LIST_ROUND) {
-            const int nc = min(LIST_ROUND, total - base), chunks = (nc + 31) >> 5;
-            __syncthreads();   // (the atoms; the round before)
-            for (int ch = wid; ch < chunks; ch += NW) {
-                const int t = ch * 32 + lane, k = base + t;
-                const bool in = t < nc;
-                float px = 0.f, py = 0.f, pz = 0.f;
-                uint32_t entry = 0;
-                int js = -1;
-                if (in) {
-                    int lo = 0, hi = nr - 1;
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (runOff[mid] <= k)
-                            lo = mid;
-                        else
-                            hi = mid - 1;
-                    }
-                    js = runSlot[lo] + (k - runOff[lo]);
-                    const int code = runShift[lo];
-                    // the candidate's image (wrapped position + w.H) relative to the origin
-                    const double4 pw = dv.posS[js];
-                    const int w0 = (code & 7) - 4, w1 = ((code >> 3) & 7) - 4, w2 = ((code >> 6) & 7) - 4;
-                    px = (float) (pw.x + (w0 * S.H[0] + w1 * S.H[3] + w2 * S.H[6]) - org.x);
-                    py = (float) (pw.y + (w1 * S.H[4] + w2 * S.H[7]) - org.y);
-                    pz = (float) (pw.z + w2 * S.H[8] - org.z);
-                    entry = (uint32_t) (js | (code << 23));
-                    cEntry[t] = entry;
-                }
-                unsigned mine = 0;
-                for (int a = 0; a < na; a++) {
-                    const float4 pa = aPos[a];
-                    const float y0 = pa.x - px, y1 = pa.y - py, y2 = pa.z - pz;
-                    const float r2 = y0 * y0 + y1 * y1 + y2 * y2;
-                    bool acc = false;
-                    if (in && js != ab + a && r2 < preF) {
-                        acc = r2 < preLoF && fabsf(y0) < hf0 && fabsf(y1) < hf1 && fabsf(y2) < hf2;
-                        if (!acc) {   // the reference's exact test on the original positions, at the image it chooses
-                            const double4 oi = dv.origS[ab + a], oj = dv.origS[js];
-                            const int4 wi = dv.wrapS[ab + a], cw = dv.wrapS[js];
-                            const double invDiag[3] = {1.0 / S.H[0], 1.0 / S.H[4], 1.0 / S.H[8]};
-                            double x[3] = {__dsub_rn(oi.x, oj.x), __dsub_rn(oi.y, oj.y), __dsub_rn(oi.z, oj.z)};
-                            int kk[3];
-                            minImageFast(x, S.H, invDiag, kk);
-                            const int w0 = (int) ((entry >> 23) & 7u) - 4, w1 = (int) ((entry >> 26) & 7u) - 4,
-                                      w2 = (int) ((entry >> 29) & 7u) - 4;
-                            acc = dot3exact(x) < S.rl2 && kk[0] - (wi.x - cw.x) == w0 && kk[1] - (wi.y - cw.y) == w1 &&
-                                  kk[2] - (wi.z - cw.z) == w2;
-                        }
-                    }
-                    const unsigned m = __ballot_sync(0xffffffffu, acc);
-                    if (lane == a)
-                        mine = m;
-                }
-                hits[ch][lane] = mine;
+    const double invDiag[3] = {1.0 / S.H[0], 1.0 / S.H[4], 1.0 / S.H[8]};
+    for (int base = 0; base < total; base += LIST_CHUNK) {
+        const int nc = min(LIST_CHUNK, total - base);
+        for (int t = tid; t < nc; t += LIST_THREADS) {
+            const int k = base + t;
+            int lo = 0, hi = nr - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (runOff[mid] <= k)
+                    lo = mid;
+                else
+                    hi = mid - 1;
             }
-            __syncthreads();
-            for (int a = wid; a < na; a += NW) {
-                const unsigned m = lane < chunks ? hits[lane][a] : 0u;
-                int v = __popc(m);
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, v, o);
-                    if (lane >= o)
-                        v += y;
-                }
-                const int count = aCount[a], first = count + v - __popc(m);
-                uint32_t* row = dv.slist + (size_t) (ab + a) * dv.cap;
-                for (unsigned some = __ballot_sync(0xffffffffu, m != 0); some; some &= some - 1) {
-                    const int ch = __ffs(some) - 1;
-                    const unsigned mc = __shfl_sync(0xffffffffu, m, ch);
-                    const int pos = __shfl_sync(0xffffffffu, first, ch) + __popc(mc & ((1u << lane) - 1u));
-                    if (((mc >> lane) & 1u) && pos < dv.cap)
-                        row[pos] = cEntry[ch * 32 + lane];
-                }
-                __syncwarp();
-                if (lane == 31)
-                    aCount[a] = count + v;
-            }
+            const int js = runSlot[lo] + (k - runOff[lo]);
+            const int code = runShift[lo];
+            const int w0 = (code & 7) - 4, w1 = ((code >> 3) & 7) - 4, w2 = ((code >> 6) & 7) - 4;
+            // the candidate's image (wrapped position + w.H) relative to the origin, staged once for the cell
+            const double4 pw = dv.posS[js];
+            cPos[t] = make_float4((float) (pw.x + (w0 * S.H[0] + w1 * S.H[3] + w2 * S.H[6]) - org.x),
+                                  (float) (pw.y + (w1 * S.H[4] + w2 * S.H[7]) - org.y),
+                                  (float) (pw.z + w2 * S.H[8] - org.z), 0.0f);
+            cEntry[t] = (uint32_t) (js | (code << 23));
         }
         __syncthreads();
-        if (tid < na) {
-            const int cnt = aCount[tid];
-            dv.slistCount[ab + tid] = min(cnt, dv.cap);
-            if (cnt > dv.cap)
-                atomicMax(&dv.flags[0], cnt);
+        for (int ii = cb + wid; ii < ce; ii += NW) {
+            const double4 pwi = dv.posS[ii];
+            const float xi = (float) (pwi.x - org.x), yi = (float) (pwi.y - org.y), zi = (float) (pwi.z - org.z);
+            uint32_t* row = dv.slist + (size_t) ii * dv.cap;
+            int count = dv.slistCount[ii];
+            for (int t0 = 0; t0 < nc; t0 += 32) {
+                const int t = t0 + lane;
+                bool acc = false, unsure = false;
+                uint32_t entry = 0;
+                if (t < nc) {
+                    const float4 pj = cPos[t];
+                    entry = cEntry[t];
+                    const float y0 = xi - pj.x, y1 = yi - pj.y, y2 = zi - pj.z;
+                    const float r2 = y0 * y0 + y1 * y1 + y2 * y2;
+                    if ((int) (entry & 0x7FFFFFu) != ii && r2 < preF) {
+                        if (r2 < preLoF && fabsf(y0) < hf0 && fabsf(y1) < hf1 && fabsf(y2) < hf2)
+                            acc = true;
+                        else
+                            unsure = true;
+                    }
+                }
+                if (__any_sync(0xffffffffu, unsure) && unsure) {
+                    // the reference's exact test on the original positions; kept only at the image it chooses
+                    const int js = (int) (entry & 0x7FFFFFu);
+                    const int w0 = (int) ((entry >> 23) & 7u) - 4, w1 = (int) ((entry >> 26) & 7u) - 4,
+                              w2 = (int) ((entry >> 29) & 7u) - 4;
+                    const double4 oi = dv.origS[ii], oj = dv.origS[js];
+                    const int4 wi = dv.wrapS[ii], cw = dv.wrapS[js];
+                    double x[3] = {__dsub_rn(oi.x, oj.x), __dsub_rn(oi.y, oj.y), __dsub_rn(oi.z, oj.z)};
+                    int kk[3];
+                    minImageFast(x, S.H, invDiag, kk);
+                    if (dot3exact(x) < S.rl2)
+                        acc = (kk[0] - (wi.x - cw.x) == w0 && kk[1] - (wi.y - cw.y) == w1 &&
+                               kk[2] - (wi.z - cw.z) == w2);
+                }
+                const unsigned ma = __ballot_sync(0xffffffffu, acc);
+                if (acc) {
+                    const int pos = count + __popc(ma & ((1u << lane) - 1u));
+                    if (pos < dv.cap)
+                        row[pos] = entry;
+                }
+                count += __popc(ma);
+            }
+            if (lane == 0)
+                dv.slistCount[ii] = count;
+        }
+        __syncthreads();
+    }
+    for (int ii = cb + tid; ii < ce; ii += LIST_THREADS) {
+        const int cnt = dv.slistCount[ii];
+        if (cnt > dv.cap) {
+            atomicMax(&dv.flags[0], cnt);
+            dv.slistCount[ii] = dv.cap;
         }
     }
 }
@@ -577,6 +558,22 @@ __global__ void k_list_from_candidates(Dev dv) {
 template <typename R> struct PairRec { static constexpr bool storeX = false; };
 template <> struct PairRec<float> { static constexpr bool storeX = true; };
 
+// x = pw_i - pw_j - w.H of the list entry e in double, rounded to R (most pairs are inside the box: w = 0).
+template <typename R>
+__device__ __forceinline__ void pairVector(double4 pwj, double4 pwi, uint32_t e, const double* H, R* x) {
+    double x0 = pwi.x - pwj.x, x1 = pwi.y - pwj.y, x2 = pwi.z - pwj.z;
+    if ((int) (e >> 23) != NO_SHIFT) {
+        double sh[3];
+        entryShift(e, H, sh);
+        x0 -= sh[0];
+        x1 -= sh[1];
+        x2 -= sh[2];
+    }
+    x[0] = (R) x0;
+    x[1] = (R) x1;
+    x[2] = (R) x2;
+}
+
 // The pair records of every listed pair (the list of the evaluation) in precision R with G0..G3 by
 // core/pgm_math.h:77-93 via pairKernels, from the current slot-order positions (also after new positions on a
 // kept list), one warp per slot, the pairs of its row over the lanes.
@@ -611,8 +608,10 @@ __global__ void __launch_bounds__(256) k_pair_kernels(Dev dv) {
         const double x0 = pwi.x - pwj.x - sh[0], x1 = pwi.y - pwj.y - sh[1], x2 = pwi.z - pwj.z - sh[2];
         const R Rj = (R) dv.radS[js], Rr = (R) Ri;
         const R xr0 = (R) x0, xr1 = (R) x1, xr2 = (R) x2;
+        const R r = fsqrt(xr0 * xr0 + xr1 * xr1 + xr2 * xr2);
+        const R a = R(1) / fsqrt(R(2) * (Rr * Rr + Rj * Rj));
         R G[4];
-        recordKernels(xr0 * xr0 + xr1 * xr1 + xr2 * xr2, R(2) * (Rr * Rr + Rj * Rj), beta, G);
+        pairKernels<R, 4>(a, beta, r, G);
         if (FIELD) {
             const R4 dj = dS[js];
             const R c = (dj.x * xr0 + dj.y * xr1 + dj.z * xr2) * G[2] + dj.w * G[1];
@@ -667,7 +666,7 @@ __global__ void __launch_bounds__(256) k_pair_kernels(Dev dv) {
 // (core/pgm_core.cpp:64-87) only near the cutoff or near half a box edge.  A pair within the cutoff whose exact
 // image is not the one stored at the build sets flags[9]: the list is rebuilt and the evaluation repeated.
 template <typename R>
-__global__ void __launch_bounds__(256, 3) k_pair_compact(Dev dv) {
+__global__ void __launch_bounds__(256, std::is_same<R, float>::value ? 4 : 3) k_pair_compact(Dev dv) {
     typedef typename V2T<R>::T R2;
     typedef typename V4T<R>::T R4;
     constexpr bool STORE_X = PairRec<R>::storeX;
@@ -689,11 +688,7 @@ __global__ void __launch_bounds__(256, 3) k_pair_compact(Dev dv) {
                  half2 = 0.5 * S.H[8] * (1.0 - 1e-10);
     // test of list entry t (t < cnt): pair geometry x and whether the pair is within the cutoff
     auto test = [&](int t, uint32_t e, double4 pwj, double* x) -> bool {
-        double sh[3];
-        entryShift(e, S.H, sh);
-        x[0] = pwi.x - pwj.x - sh[0];
-        x[1] = pwi.y - pwj.y - sh[1];
-        x[2] = pwi.z - pwj.z - sh[2];
+        pairVector(pwj, pwi, e, S.H, x);
         const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
         if (!(r2 < pre))
             return false;
@@ -769,8 +764,10 @@ __global__ void __launch_bounds__(256, 3) k_pair_compact(Dev dv) {
             xr2 = (R) (pwi.z - pwj.z - sh[2]);
         }
         const R Rj = (R) dv.radS[js];
+        const R r = fsqrt(xr0 * xr0 + xr1 * xr1 + xr2 * xr2);
+        const R a = R(1) / fsqrt(R(2) * (Rr * Rr + Rj * Rj));
         R G[4];
-        recordKernels(xr0 * xr0 + xr1 * xr1 + xr2 * xr2, R(2) * (Rr * Rr + Rj * Rj), beta, G);
+        pairKernels<R, 4>(a, beta, r, G);
         R2 vb;
         if constexpr (STORE_X) {
             va.w = G[1];
@@ -792,7 +789,7 @@ __global__ void __launch_bounds__(256, 3) k_pair_compact(Dev dv) {
 // ------------------------------------------------------------------------------------------------ dipoles
 
 // Permanent dipoles p_i = sum_m c_m unit(minimage(r_partner - r_atom)) over the dipoles of atom i
-// (core/pgm_core.cpp:51-62).
+// (core/pgm_core.cpp:51-62), and each dipole's geometry in the order that the forces' chain rule reads it.
 __global__ void k_perm(Dev dv) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= dv.nAtoms)
