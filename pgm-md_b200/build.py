@@ -19,7 +19,7 @@ PKG = Path(__file__).resolve().parent
 ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libpgm_b200.so"
-SOURCES = [CSRC / "engine.cu", CSRC / "transforms.cu", CSRC / "persistent.cu",
+SOURCES = [CSRC / "engine.cu", CSRC / "transforms.cu", CSRC / "transforms64.cu", CSRC / "persistent.cu",
            CSRC / "capi.cpp"]
 HEADERS = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [ROOT / "include" / "pgm_b200.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -182,9 +182,9 @@ struct Engine::Impl {
     // TF_GRID one cooperative kernel, a block per x-plane
     // TF_PCG the grid kernel for the field passes outside the CG loop, and the whole CG loop as one persistent
     //   cooperative kernel (mixed precision, one system)
-    enum { TF_CUFFT = 0, TF_CLUSTER = 1, TF_SPLIT = 2, TF_GRID = 3, TF_PCG = 4 };
+    enum { TF_AUTO = -1, TF_CUFFT = 0, TF_CLUSTER = 1, TF_SPLIT = 2, TF_GRID = 3, TF_PCG = 4 };
     int tfMode = TF_CUFFT;     // in use
-    int tfWant = TF_CUFFT;     // the caller's choice (setTransforms)
+    int tfWant = TF_AUTO;      // the caller's choice (setTransforms), or the rule of selectTransforms
     bool fuseCgA = true;       // single system: A p and alph in the CG gather's epilogue (else a separate kernel)
     bool clusterOk = false;    // the systems' grids and the GPU allow the cluster kernel
     bool splitOk = false;      // the systems' x extents allow the x-line kernel
@@ -199,7 +199,6 @@ struct Engine::Impl {
     int pcgBlocks = 0;         // its blocks (one per SM)
     size_t pcgSmem = 0;
     int fftcBuf = 0, fftcC = 16, fftgBuf = 0, maxK0 = 0;
-    int pcgKc = 0;             // the one system's grid is pcgKc^3, or 0
     int fftgKc = 0;            // the grid transforms' compile-time size (every grid fftgKc^3), or 0
     size_t fftgSmem = 0;
     int maxLineBlocks = 0;
@@ -365,7 +364,7 @@ struct Engine::Impl {
         CU(cudaMallocHost((void**) &hCtl, sizeof(Ctl)));
         useGraph = envInt("PGM_B200_NO_GRAPH", 0) == 0;
         pairGS = envInt("PGM_B200_PAIR_LANES", 32);
-        tfWant = envInt("PGM_B200_TRANSFORMS", TF_CUFFT);
+        tfWant = envInt("PGM_B200_TRANSFORMS", TF_AUTO);
         fuseCgA = envInt("PGM_B200_FUSED_CG", 1) != 0;
         // the field pair pass runs beside the transforms of the same pass: optionally at most pairBlocks of its
         // blocks per SM (a shared-memory reservation it does not use), so that the transform kernels find room
@@ -645,8 +644,7 @@ struct Engine::Impl {
             for (int k = 0; k < nsys; k++)
                 for (int a = 0; a < 3; a++)
                     fftgKc = sysK[k][a] == fftgKc ? fftgKc : 0;
-            pcgKc = fftgKc;
-            if (fftgKc != 32 && fftgKc != 40 && fftgKc != 48 && fftgKc != 64)
+            if (fftgKc < FFTG_MIN_K)
                 fftgKc = 0;
         }
         if (clusterOk) {
@@ -1213,7 +1211,7 @@ struct Engine::Impl {
         pcgSmem = pcgSmemBytes((n + pcgBlocks - 1) / pcgBlocks, fftgBuf);
         if (!coop || pcgSmem > (size_t) optin || K[0] + PCG_MIN_PAIR_BLOCKS > pcgBlocks)
             return;
-        PcgKernel kfn = pcgKernel(pcgKc);
+        PcgKernel kfn = pcgKernel(fftgKc);
         CU(cudaFuncSetAttribute((const void*) kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) pcgSmem));
         int perSm = 0;
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kfn, PCG_THREADS, pcgSmem));
@@ -1365,7 +1363,7 @@ struct Engine::Impl {
     // The whole CG solve after the permanent field (or for the right-hand side in b): one cooperative launch of the
     // persistent kernel (one block per SM).
     void launchPersistent(cudaStream_t sm, const Dev& d) {
-        PcgKernel kfn = pcgKernel(pcgKc);
+        PcgKernel kfn = pcgKernel(fftgKc);
         CU(cudaFuncSetAttribute((const void*) kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) pcgSmem));
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[1];
@@ -1410,9 +1408,22 @@ struct Engine::Impl {
     void tangentPass(const Dev& d, const FmBufs& B, const double* dr, const double* dd, const double* dip,
                      const double* quadD, int withQ);
 
-    // The transform mode in use: the caller's choice where the systems' grids allow it, else cuFFT.
+    // The transform mode in use: the caller's choice where the systems' grids allow it, else cuFFT.  Until the caller
+    // chooses, one system takes the persistent kernel (with its own spread and gather, so not when the caller chose
+    // other PME kernels or the dual first pass), else the grid kernel where it is compiled for the grid.  Measured on one
+    // B200, us an evaluation, persistent / grid kernel / cuFFT: mixed 72 atoms (9^3) 252 / 384 / 357, 648 (20^3) 285 / 422
+    // / 417, 4113 (36^3) 420 / 562 / 562, 8550 (48^3) 593 / 717 / 929, 12288 (50^3) 705 / 917 / 877; FP64 93 (48^3) - / 364
+    // / 447, 8550 (48^3) - / 945 / 1039, but 648 (20^3, the general grid kernel) - / 423 / 410.  Batches keep cuFFT, whose plans
+    // take all systems of a shape at once.
     void selectTransforms() {
         int m = TF_CUFFT;
+        if (tfWant == TF_AUTO && nsys == 1) {
+            const char* dual = std::getenv("PGM_B200_DUAL");
+            if (pcgOk && pmeWant == 0 && !(dual && dual[0] == '1'))
+                m = TF_PCG;
+            else if (gridOk && fftgKc > 0)
+                m = TF_GRID;
+        }
         if (tfWant == TF_CLUSTER && clusterOk)
             m = TF_CLUSTER;
         if (tfWant == TF_SPLIT && splitOk)
@@ -3146,6 +3157,7 @@ void Engine::setPmeKernels(int kind) {
         I.exec = nullptr;
     }
     I.pmeWant = kind;
+    I.selectTransforms();   // (the rule without a caller's choice depends on it)
 }
 
 int Engine::pmeKernels() const {

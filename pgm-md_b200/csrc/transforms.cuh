@@ -1,12 +1,14 @@
-// The cooperative kernels compiled in a translation unit of their own (transforms.cu).
+// The cooperative kernels compiled in translation units of their own.
 #pragma once
 
 #include "common.cuh"
 
 namespace pgmb200 {
 
-// The grid-transform kernel: compiled for one cubic grid size (32, 40, 48, 64), or for any grid (kc = 0); energy: the
-// final pass's variant that also sums the reciprocal energy and strain.
+// The grid-transform kernel, compiled for every cubic 2-3-5 grid of 8 to 64 points (the general kernel's run-time radices and
+// index divisions cost it 6 us at 30^3), any other grid by the general one (kc = 0); energy: the final pass's variant that
+// also sums the reciprocal energy and strain.
+constexpr int FFTG_MIN_K = 8;
 typedef void (*GridKernel)(Dev, int);
 template <typename R> GridKernel gridKernel(int kc, bool energy);
 
