@@ -170,6 +170,13 @@ struct Dev {
     const int* covByAtom;
     const int* covByPartnerOff;
     const int* covByPartner;
+    const int* covPartnerPos; // the place of each dipole in covByPartner
+    // the evaluation's dipoles (k_perm): by atom's row (unit vector, strength / length) and length, by partner's row the
+    // same with the dipole's atom
+    double4* covOwn;
+    double* covOwnLen;
+    double4* covOther;
+    int* covOtherAtom;
     // chunks
     const int* chunkSys;
     const int* chunkBegin;

@@ -211,7 +211,7 @@ struct Engine::Impl {
         dDS2, dEpair2, dErec2, dGrid2, dGridFix, dGridFix2,
         dScal, dPartial, dGPartial, dHrec, dFm, dPmeRec, dPmeBins, dSrcW, dGPart, dPcgPartial, dBinCount, dActive, dActSys, dSysCounter, dEpair, dErec, dFpair, dSpair, dFrec, dEtot, dFin, dPot, dForces, dResults,
         dConvPartial, dConvOff, dGrid, dSpec, dInfl, dTwiddle, dModuli, dCovAtom, dCovPartner, dCovStrength, dCovByAtomOff,
-        dCovByAtom, dCovByPartnerOff, dCovByPartner, dChunkSys, dChunkBegin, dChunkEnd, dHist, dGlobal, dCtl,
+        dCovByAtom, dCovByPartnerOff, dCovByPartner, dCovPartnerPos, dCovOwn, dCovOwnLen, dCovOther, dCovOtherAtom, dChunkSys, dChunkBegin, dChunkEnd, dHist, dGlobal, dCtl,
         dGradQ, dGradR, dSList, dSListCount, dPosBuild, dAtomSlot, dCandStart, dCandJ, dCandT, dGv, dSkipStart, dSkipJ;
     // FP64 shadow of the mixed path for the iterative refinement
     Buf dPairBd, dDSd, dGridD, dSpecD, dInflD, dSplD, dB64, dXsave;
@@ -521,6 +521,14 @@ struct Engine::Impl {
             byAtom[fa[covAtom[m]]++] = m;
             byPartner[fp[covPartner[m]]++] = m;
         }
+        std::vector<int> partnerPos(ncov);   // the place of each dipole among the partners' rows
+        for (int k = 0; k < ncov; k++)
+            partnerPos[byPartner[k]] = k;
+        upload(dCovPartnerPos, partnerPos, st);
+        dCovOwn.ensure(std::max(ncov, 1) * sizeof(double4));
+        dCovOwnLen.ensure(std::max(ncov, 1) * 8);
+        dCovOther.ensure(std::max(ncov, 1) * sizeof(double4));
+        dCovOtherAtom.ensure(std::max(ncov, 1) * sizeof(int));
         upload(dCovAtom, covAtom, st);
         upload(dCovPartner, covPartner, st);
         upload(dCovStrength, covStrength, st);
@@ -1095,6 +1103,11 @@ struct Engine::Impl {
         d.covByAtom = dCovByAtom.as<int>();
         d.covByPartnerOff = dCovByPartnerOff.as<int>();
         d.covByPartner = dCovByPartner.as<int>();
+        d.covPartnerPos = dCovPartnerPos.as<int>();
+        d.covOwn = dCovOwn.as<double4>();
+        d.covOwnLen = dCovOwnLen.as<double>();
+        d.covOther = dCovOther.as<double4>();
+        d.covOtherAtom = dCovOtherAtom.as<int>();
         d.chunkSys = dChunkSys.as<int>();
         d.chunkBegin = dChunkBegin.as<int>();
         d.chunkEnd = dChunkEnd.as<int>();
@@ -1403,6 +1416,13 @@ struct Engine::Impl {
                 break;
         }
     }
+    // The grid cleared for a spread that adds to it (the fixed-point spread leaves the float grid to the transforms, which
+    // write every point).
+    template <typename R> void clearGrid(cudaStream_t sm, const Dev& d) {
+        if (!(std::is_same<R, float>::value && d.gridFix))
+            CU(cudaMemsetAsync(d.grid, 0, gridTotal * sizeof(R), sm));
+    }
+
     int solveDevice(double tol);
     template <typename R>
     void tangentPass(const Dev& d, const FmBufs& B, const double* dr, const double* dd, const double* dip,
@@ -1638,10 +1658,11 @@ struct Engine::Impl {
         CU(cudaGetLastError());
     }
 
-    // The first half of a build: wraps, cells and the slot order with its slot-order copies.
-    void enqueueCells(cudaStream_t sm, const Dev& d) {
+    // The first half of a build: wraps, cells and the slot order with its slot-order copies (prep 2; 3: also the
+    // evaluation's positions in, in the same kernel).
+    void enqueueCells(cudaStream_t sm, const Dev& d, int prep = 2) {
         const int tb = (n + 255) / 256;
-        k_prep<<<tb, 256, 0, sm>>>(d, nullptr, 2);
+        k_prep<<<tb, 256, 0, sm>>>(d, (prep & 1) ? dPosIn.as<double>() : nullptr, prep);
         k_cell_scan<<<1, 1024, 0, sm>>>(d);
         k_cell_scatter<<<tb, 256, 0, sm>>>(d);
         k_cell_sort<<<(totalCells + 7) / 8, 256, 0, sm>>>(d);
@@ -1658,20 +1679,20 @@ struct Engine::Impl {
 
     // The pair-list step of an evaluation: positions in (PME base and fraction), the stale test, the build when
     // stale (a conditional node of the graph, its body captured after the main capture; without graphs a host
-    // decision), the slot-order positions with the build's wraps.  Without a skin the list's rows are left to the
-    // caller (listKernel after this step, on a stream of its choice: nothing before it reads the list; the
-    // refreshed slot copies equal the cell sort's bit for bit), and the call returns true.
+    // decision), the slot-order positions with the build's wraps.  Without a skin the cell sort has just written
+    // those (the same bits), and the list's rows are left to the caller (listKernel after this step, on a stream of its
+    // choice: nothing before it reads the list); the call returns true.
     bool enqueueListStep(cudaStream_t sm, const Dev& d) {
-        const int tb = (n + 255) / 256;
-        k_prep<<<tb, 256, 0, sm>>>(d, dPosIn.as<double>(), 1);
         const bool rowsLeft = !verletList();
         if (rowsLeft) {   // no skin: a build at every evaluation, without the stale test or a conditional node
             CU(cudaMemsetAsync(d.cellCount, 0, (size_t) totalCells * sizeof(int), sm));
-            enqueueCells(sm, d);
+            enqueueCells(sm, d, 3);
         } else {
+            const int tb = (n + 255) / 256;
+            k_prep<<<tb, 256, 0, sm>>>(d, dPosIn.as<double>(), 1);
             enqueueStaleBuild(sm, d);
+            k_refresh_positions<<<tb, 256, 0, sm>>>(d);
         }
-        k_refresh_positions<<<tb, 256, 0, sm>>>(d);
         CU(cudaGetLastError());
         return rowsLeft;
     }
@@ -1737,7 +1758,7 @@ struct Engine::Impl {
                     enqueuePlaneBins(sd, d);
                 k_perm<<<tb, 256, 0, sd>>>(d);
                 k_influence<R><<<dim3(convBlocks, nsys), 256, 0, sd>>>(d);
-                CU(cudaMemsetAsync(d.grid, 0, gridTotal * realSize(), sd));
+                clearGrid<R>(sd, d);
                 launchSpread<R>(sd, d, 0, d.perm);
                 CU(cudaEventRecord(evPerm, sd));
                 transformPair<R>(sd, d, false, spreadFix());
@@ -1757,12 +1778,12 @@ struct Engine::Impl {
                     return;
                 k_cg_b<<<(int) chunkSys.size(), CHUNK, 0, sm>>>(d);
                 CU(cudaGetLastError());
-                CU(cudaMemsetAsync(d.grid, 0, gridTotal * realSize(), sm));
+                clearGrid<R>(sm, d);
                 fieldPass<R, false>(sm, sd, d, 1, d.x, false);
                 k_cg_init<<<(int) chunkSys.size(), CHUNK, 0, sm>>>(d);
                 CU(cudaGetLastError());
                 // the loop's first spread needs a clear grid (each iteration clears it for the next one)
-                CU(cudaMemsetAsync(d.grid, 0, gridTotal * realSize(), sm));
+                clearGrid<R>(sm, d);
                 return;
             }
             // a predicted step (dualFirstPass): x0 from the history first; (q, perm) into the grid and dS, x0 into
@@ -1782,8 +1803,8 @@ struct Engine::Impl {
             k_perm<<<tb, 256, 0, sd>>>(d);
             k_influence<R><<<dim3(convBlocks, nsys), 256, 0, sd>>>(d);
             k_cg_guess<<<(3 * n + 255) / 256, 256, 0, sd>>>(d);
-            CU(cudaMemsetAsync(d.grid, 0, gridTotal * realSize(), sd));
-            CU(cudaMemsetAsync(d2.grid, 0, gridTotal * realSize(), sd));
+            clearGrid<R>(sd, d);
+            clearGrid<R>(sd, d2);
             launchSpread<R>(sd, d, 0, d.perm);
             launchSpread<R>(sd, d2, 1, d.x);
             CU(cudaEventRecord(evPerm, sd));
@@ -1804,7 +1825,7 @@ struct Engine::Impl {
             d3.Erec = dErec2.as<double>();
             k_cg_init<<<(int) chunkSys.size(), CHUNK, 0, sm>>>(d3);
             CU(cudaGetLastError());
-            CU(cudaMemsetAsync(d.grid, 0, gridTotal * realSize(), sm));
+            clearGrid<R>(sm, d);
         } else {
             if (rowsLeft)
                 listKernel(sm, d);
@@ -1837,7 +1858,7 @@ struct Engine::Impl {
 
     template <typename R> void enqueuePost(cudaStream_t sm, cudaStream_t sd, const Dev& d) {
         const int tb = (n + 255) / 256;
-        CU(cudaMemsetAsync(d.grid, 0, gridTotal * realSize(), sm));
+        clearGrid<R>(sm, d);
         k_final_prep<<<tb, 256, 0, sm>>>(d, s.polarizable ? 1 : 0);
         launchSpread<R>(sm, d, 0, d.dtot);
         CU(cudaEventRecord(evFork, sm));
@@ -1863,7 +1884,6 @@ struct Engine::Impl {
         CU(cudaEventRecord(evJoin, sd));
         CU(cudaStreamWaitEvent(sm, evJoin, 0));
         launchGather<R, true>(sm, d, 0);
-        k_final_field<<<tb, 256, 0, sm>>>(d);
         k_final_forces<<<(int) chunkSys.size(), CHUNK, 0, sm>>>(d, s.polarizable ? 1 : 0);
         CU(cudaGetLastError());
     }
@@ -2617,14 +2637,14 @@ void Engine::field(const double* pos, const double box[3][3], const double* qf, 
             k_pair_compact<float><<<(I.n + 7) / 8, 256, 0, I.st>>>(dv);
             k_splines<float><<<(3 * I.n + 255) / 256, 256, 0, I.st>>>(dv);
             k_influence<float><<<dim3(I.convBlocks, I.nsys), 256, 0, I.st>>>(dv);
-            CU(cudaMemsetAsync(dv.grid, 0, I.gridTotal * I.realSize(), I.st));
+            I.clearGrid<float>(I.st, dv);
             I.fieldPass<float, true>(I.st, I.side, dv, 0, dv.dtot, false);
         } else {
             I.listKernel(I.st, dv);
             k_pair_compact<double><<<(I.n + 7) / 8, 256, 0, I.st>>>(dv);
             k_splines<double><<<(3 * I.n + 255) / 256, 256, 0, I.st>>>(dv);
             k_influence<double><<<dim3(I.convBlocks, I.nsys), 256, 0, I.st>>>(dv);
-            CU(cudaMemsetAsync(dv.grid, 0, I.gridTotal * I.realSize(), I.st));
+            I.clearGrid<double>(I.st, dv);
             I.fieldPass<double, true>(I.st, I.side, dv, 0, dv.dtot, false);
         }
         CU(cudaGetLastError());
@@ -2811,10 +2831,10 @@ int Engine::Impl::solveDevice(double tol) {
             return;
         }
         k_cg_b<<<(int) chunkSys.size(), CHUNK, 0, st>>>(d);
-        CU(cudaMemsetAsync(d.grid, 0, gridTotal * realSize(), st));
+        clearGrid<R>(st, d);
         fieldPass<R, false>(st, side, d, 1, d.x, false);
         k_cg_init<<<(int) chunkSys.size(), CHUNK, 0, st>>>(d);
-        CU(cudaMemsetAsync(d.grid, 0, gridTotal * realSize(), st));
+        clearGrid<R>(st, d);
         solveLoop<R>(d);
     };
     if (mixed())
@@ -2976,10 +2996,10 @@ int Engine::solve(const double* rhs, double* x, double tol) {
             return;
         }
         k_cg_b<<<(int) I.chunkSys.size(), CHUNK, 0, I.st>>>(d);
-        CU(cudaMemsetAsync(d.grid, 0, I.gridTotal * I.realSize(), I.st));
+        I.clearGrid<R>(I.st, d);
         I.fieldPass<R, false>(I.st, I.side, d, 1, d.x, false);
         k_cg_init<<<(int) I.chunkSys.size(), CHUNK, 0, I.st>>>(d);
-        CU(cudaMemsetAsync(d.grid, 0, I.gridTotal * I.realSize(), I.st));
+        I.clearGrid<R>(I.st, d);
         I.solveLoop<R>(d);
     };
     if (I.mixed())
@@ -3013,18 +3033,17 @@ int Engine::kernelLaunches() const {
     const Impl& I = *impl;
     if (!I.haveResult)
         return 0;
-    // own kernels per evaluation (the cuFFT transforms not counted): preparation 7, the Verlet list's build 5
-    // when it ran; a field pass fp = 4 (spread, the cluster transform kernel or the influence product, pair
-    // pass, gather); polarizable: two field passes + 2 before the loop, fp + 2 per CG iteration (fp + 1 for one
-    // system); final 7
+    // own kernels per evaluation (the cuFFT transforms not counted): with a kept list preparation 7 and the Verlet
+    // list's build 5 when it ran, without a skin 9; a field pass fp = 4 (spread, the transform kernel or the influence
+    // product, pair pass, gather); polarizable: two field passes + 2 before the loop, fp + 2 per CG iteration (fp + 1 with
+    // A p in the gather), or one pass and one launch for the whole solve; final 6
     int it = 0;
     for (int k = 0; k < I.nsys; k++)
         it = std::max(it, (int) I.lastResults[(size_t) k * NRES + 14]);
-    const int fp = 4;
-    const int perIt = fp + (I.fusedGather() ? 1 : 2);   // single system: A p in the gather
-    if (I.persistentMode() && I.s.polarizable)   // the permanent field's pass and one launch for the whole solve
-        return 7 + (I.lastBuilt ? 5 : 0) + fp + 1 + 7 + (I.gvdwOn ? 1 : 0);
-    return 7 + (I.lastBuilt ? 5 : 0) + (I.s.polarizable ? 2 * fp + 2 + perIt * it : 0) + 7 + (I.gvdwOn ? 1 : 0);
+    const int fp = 4, perIt = fp + (I.fusedGather() ? 1 : 2);
+    const int pre = I.verletList() ? 7 + (I.lastBuilt ? 5 : 0) : 9;
+    const int solve = !I.s.polarizable ? 0 : I.persistentMode() ? fp + 1 : 2 * fp + 2 + perIt * it;
+    return pre + solve + 6 + (I.gvdwOn ? 1 : 0);
 }
 
 void Engine::kernelTimes(int reps, double* ms, void* flush, size_t flushBytes) {

@@ -806,6 +806,12 @@ __global__ void k_perm(Dev dv) {
         const double L = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
         for (int a = 0; a < 3; a++)
             p[a] += dv.covStrength[m] * v[a] / L;
+        const double4 u = make_double4(v[0] / L, v[1] / L, v[2] / L, dv.covStrength[m] / L);
+        const int at = dv.covPartnerPos[m];
+        dv.covOwn[k] = u;
+        dv.covOwnLen[k] = L;
+        dv.covOther[at] = u;
+        dv.covOtherAtom[at] = i;
     }
     for (int a = 0; a < 3; a++)
         dv.perm[3 * i + a] = p[a];
@@ -1523,6 +1529,9 @@ __device__ __forceinline__ void gatherSlot(const Dev& dv, const SysDev& S, int s
         dv.Erec[3 * i + k] = E;
         if (FINAL) {
             const double* d = dv.dtot + 3 * i;
+            // the total field E = E_pair + E_rec + cs d (core/pgm_core.cpp:437-438, 445-448, 494-495)
+            const double cs = 4.0 * S.beta * S.beta * S.beta / (3.0 * SQRT_PI);
+            dv.Etot[3 * i + k] = dv.Epair[3 * i + k] + E + cs * d[k];
             double e[3];
             for (int a = 0; a < 3; a++)
                 e[a] = S.K[a] * (d[0] * S.recip[a] + d[1] * S.recip[3 + a] + d[2] * S.recip[6 + a]);
@@ -2216,30 +2225,14 @@ __global__ void k_final_prep(Dev dv, int solved) {
     dv.fin[(size_t) i * NFIN + 2] = (al > 0) ? m2 / (2.0 * al) : 0.0;
 }
 
-// Total field E = E_pair + E_rec + cs d (core/pgm_core.cpp:437-438, 445-448, 494-495).
-__global__ void k_final_field(Dev dv) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= dv.nAtoms)
-        return;
-    const SysDev& S = dv.sys[dv.atomSys[i]];
-    const double cs = 4.0 * S.beta * S.beta * S.beta / (3.0 * SQRT_PI);
-    for (int k = 0; k < 3; k++)
-        dv.Etot[3 * i + k] = dv.Epair[3 * i + k] + dv.Erec[3 * i + k] + cs * dv.dtot[3 * i + k];
-}
-
-__device__ __forceinline__ void covalentTerm(const Dev& dv, const SysDev& S, int m, double* t, double* v) {
-    const int i = dv.covAtom[m], j = dv.covPartner[m];
-    v[0] = dv.posIn[3 * j] - dv.posIn[3 * i];
-    v[1] = dv.posIn[3 * j + 1] - dv.posIn[3 * i + 1];
-    v[2] = dv.posIn[3 * j + 2] - dv.posIn[3 * i + 2];
-    int kk[3];
-    minImageExact(v, S.H, kk);
-    const double L = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-    const double u[3] = {v[0] / L, v[1] / L, v[2] / L};
-    const double g[3] = {-dv.Etot[3 * i], -dv.Etot[3 * i + 1], -dv.Etot[3 * i + 2]};
-    const double gu = g[0] * u[0] + g[1] * u[1] + g[2] * u[2];
-    for (int k = 0; k < 3; k++)
-        t[k] = dv.covStrength[m] * (g[k] - gu * u[k]) / L;
+// The chain rule of one covalent dipole with atom i (unit vector u, cL = strength / length): t = cL (g - (g.u) u), g =
+// -E_tot(i).
+__device__ __forceinline__ void covalentTerm(const Dev& dv, double4 u, int i, double* t) {
+    const double g0 = -dv.Etot[3 * i], g1 = -dv.Etot[3 * i + 1], g2 = -dv.Etot[3 * i + 2];
+    const double gu = g0 * u.x + g1 * u.y + g2 * u.z;
+    t[0] = u.w * (g0 - gu * u.x);
+    t[1] = u.w * (g1 - gu * u.y);
+    t[2] = u.w * (g2 - gu * u.z);
 }
 
 // Forces F = ke (pair + reciprocal + covalent chain rule, core/pgm_core.cpp:511-535), written to the
@@ -2261,9 +2254,13 @@ __global__ void __launch_bounds__(CHUNK) k_final_forces(Dev dv, int iterationsSo
         double Sv[9];
         for (int k = 0; k < 9; k++)
             Sv[k] = dv.spair[(size_t) i * 9 + k] + dv.fin[(size_t) i * NFIN + 3 + k];
+        // the dipoles' geometry lies in row order (k_perm), so a term costs a load and its arithmetic, not a chain of
+        // indices, two positions, a square root and divisions (a latency chain at any size: this and the fused launches around it take 10 to 25 us off an evaluation)
         for (int c = dv.covByAtomOff[i]; c < dv.covByAtomOff[i + 1]; c++) {
-            double t[3], vv[3];
-            covalentTerm(dv, S, dv.covByAtom[c], t, vv);
+            double t[3];
+            const double4 u = dv.covOwn[c];
+            const double L = dv.covOwnLen[c], vv[3] = {u.x * L, u.y * L, u.z * L};
+            covalentTerm(dv, u, i, t);
             for (int k = 0; k < 3; k++) {
                 F[k] += t[k];
                 for (int b = 0; b < 3; b++)
@@ -2271,8 +2268,8 @@ __global__ void __launch_bounds__(CHUNK) k_final_forces(Dev dv, int iterationsSo
             }
         }
         for (int c = dv.covByPartnerOff[i]; c < dv.covByPartnerOff[i + 1]; c++) {
-            double t[3], vv[3];
-            covalentTerm(dv, S, dv.covByPartner[c], t, vv);
+            double t[3];
+            covalentTerm(dv, dv.covOther[c], dv.covOtherAtom[c], t);
             for (int k = 0; k < 3; k++)
                 F[k] -= t[k];
         }
