@@ -307,7 +307,8 @@ struct Engine::Impl {
                       &dPcgPartial, &dBinCount, &dActive, &dActSys, &dSysCounter, &dEpair,
                       &dErec, &dFpair, &dSpair, &dFrec, &dEtot, &dFin, &dPot, &dForces, &dResults, &dConvPartial,
                       &dConvOff, &dGrid, &dSpec, &dInfl, &dTwiddle, &dModuli, &dCovAtom, &dCovPartner, &dCovStrength,
-                      &dCovByAtomOff, &dCovByAtom, &dCovByPartnerOff, &dCovByPartner, &dChunkSys, &dChunkBegin,
+                      &dCovByAtomOff, &dCovByAtom, &dCovByPartnerOff, &dCovByPartner, &dCovPartnerPos, &dCovOwn,
+                      &dCovOwnLen, &dCovOther, &dCovOtherAtom, &dChunkSys, &dChunkBegin,
                       &dChunkEnd, &dHist, &dGlobal, &dCtl, &dGradQ, &dGradR, &dPairBd, &dDSd, &dGridD, &dSpecD,
                       &dInflD, &dSplD, &dB64, &dXsave, &dSList, &dSListCount, &dPosBuild, &dAtomSlot, &dCandStart,
                       &dCandJ, &dCandT, &dGv, &dSkipStart, &dSkipJ};
