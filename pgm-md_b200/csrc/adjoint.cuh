@@ -29,8 +29,23 @@ struct FmBufs {
     double* gR;       // n  assembled dR part
     double* ga;       // n  assembled dalpha part
     double* gc;       // ncov assembled dc part
+    double* loss;     // one per block of k_fm_target: its part of sum |F - F_target|^2
     double* Ed;       // 3n the pass's total-field derivative (D_w E_tot, or the field of u)
 };
+
+// w = 2 (F - F_target) from the evaluation's forces and the target in w, and the blocks' parts of the loss (fixed order).
+__global__ void __launch_bounds__(256) k_fm_target(Dev dv, FmBufs B) {
+    const size_t m = 3 * (size_t) dv.nAtoms;
+    double v[1] = {0.0};
+    for (size_t k = (size_t) blockIdx.x * 1024 + threadIdx.x; k < min(m, ((size_t) blockIdx.x + 1) * 1024); k += 256) {
+        const double r = dv.forces[k] - B.w[k];
+        v[0] += r * r;
+        B.w[k] = 2.0 * r;
+    }
+    blockReduce<1>(v, 0u);
+    if (threadIdx.x == 0)
+        B.loss[blockIdx.x] = v[0];
+}
 
 // D_w p_i = sum_m c_m D u_m over the covalent dipoles of atom i, D u = (dv - u (u . dv)) / L, dv = w_partner - w_atom
 // (the bond vector's change), u and L of the minimum image (core/pgm_core.cpp:51-62 differentiated).
@@ -280,7 +295,8 @@ __global__ void k_fm_assemble_w(Dev dv, FmBufs B) {
     B.ga[i] = 0.0;
 }
 
-// The pass along u (positions fixed, dipoles changed by u): dq, dR, dalpha parts and the total field of u.
+// The pass along u (positions fixed, dipoles changed by u): the total field of u, and dq, dR, dalpha less the pass along w's
+// parts, the gradients.
 __global__ void k_fm_assemble_u(Dev dv, FmBufs B, const double* u) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= dv.nAtoms)
@@ -293,13 +309,13 @@ __global__ void k_fm_assemble_u(Dev dv, FmBufs B, const double* u) {
         mu_u += dv.mu[3 * i + k] * u[3 * i + k];
     }
     const double al = dv.alpha[i];
-    B.gq[i] = dv.ke * (B.pphi[i] + B.tphi[i]);
-    B.gR[i] = dv.ke * B.pR[i];
+    B.gq[i] = dv.ke * (B.pphi[i] + B.tphi[i]) - B.gq[i];
+    B.gR[i] = dv.ke * B.pR[i] - B.gR[i];
     B.ga[i] = al > 0 ? -dv.ke * mu_u / (al * al) : 0.0;
 }
 
 // Per covalent dipole m (atom i, partner j, unit u, length L): along w, dc = -ke (D_w E_tot(i) . u + E_tot(i) . D u);
-// along u (alongW = 0), dc = -ke E_u(i) . u.
+// along u (alongW = 0), dc = -ke E_u(i) . u less that, the gradient.
 __global__ void k_fm_cov(Dev dv, FmBufs B, int alongW) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= dv.ncov)
@@ -321,7 +337,7 @@ __global__ void k_fm_cov(Dev dv, FmBufs B, int alongW) {
         for (int k = 0; k < 3; k++)
             g += dv.Etot[3 * i + k] * (dvv[k] - ud * u[k]) / L;
     }
-    B.gc[m] = -dv.ke * g;
+    B.gc[m] = alongW ? -dv.ke * g : -dv.ke * g - B.gc[m];
 }
 
 // b = -D_w E_tot (the adjoint's right-hand side).

@@ -220,11 +220,12 @@ struct Engine::Impl {
     double* hPos = nullptr;
     float* hPosF = nullptr;
     double* hForces = nullptr;
+    double* hFm = nullptr;      // the force-matching gradients' staging
     double* hResults = nullptr;
     int* hFlags = nullptr;
     Ctl* hCtl = nullptr;
     SysDev* hSys = nullptr;
-    size_t hPosCap = 0, hSysCap = 0, hResCap = 0;
+    size_t hPosCap = 0, hSysCap = 0, hResCap = 0, hFmCap = 0;
 
     // graph
     cudaGraphExec_t exec = nullptr;
@@ -317,6 +318,7 @@ struct Engine::Impl {
         if (hPos) cudaFreeHost(hPos);
         if (hPosF) cudaFreeHost(hPosF);
         if (hForces) cudaFreeHost(hForces);
+        if (hFm) cudaFreeHost(hFm);
         if (hResults) cudaFreeHost(hResults);
         if (hFlags) cudaFreeHost(hFlags);
         if (hCtl) cudaFreeHost(hCtl);
@@ -324,6 +326,8 @@ struct Engine::Impl {
         hPos = nullptr;
         hPosF = nullptr;
         hForces = nullptr;
+        hFm = nullptr;
+        hFmCap = 0;
         hResults = nullptr;
         hFlags = nullptr;
         hCtl = nullptr;
@@ -2884,9 +2888,9 @@ double Engine::forceMatchingGrad(const double* fTarget, double tol, double* dq, 
         throw std::invalid_argument("pgm_b200: forceMatchingGrad needs the target forces and tol > 0");
     I.selectDevice();
     const size_t n = I.n, ncov = I.covAtom.size();
-    // buffers: w, dp, pphi, pE, pR, tphi, tE, gq, gR, ga, gc, Ed
-    const size_t words = 3 * n + 3 * n + n + 3 * n + n + n + 3 * n + n + n + n + std::max<size_t>(ncov, 1) + 3 * n;
-    I.dFm.ensure(words * 8);
+    // buffers: w, dp, pphi, pE, pR, tphi, tE, Ed, and what goes back to the host in one piece: gq, gR, ga, gc, loss parts
+    const size_t parts = (3 * n + 1023) / 1024, nc = std::max<size_t>(ncov, 1), back = 3 * n + nc + parts;
+    I.dFm.ensure((18 * n + back) * 8);
     double* base = I.dFm.as<double>();
     FmBufs B;
     size_t off = 0;
@@ -2902,35 +2906,27 @@ double Engine::forceMatchingGrad(const double* fTarget, double tol, double* dq, 
     B.pR = take(n);
     B.tphi = take(n);
     B.tE = take(3 * n);
+    B.Ed = take(3 * n);
     B.gq = take(n);
     B.gR = take(n);
     B.ga = take(n);
-    B.gc = take(std::max<size_t>(ncov, 1));
-    B.Ed = take(3 * n);
-    // w = 2 (F - F_target) and the loss, on the host (the forces of the last evaluation)
-    std::vector<double> F(3 * n), w(3 * n);
-    CU(cudaMemcpyAsync(F.data(), I.dForces.p, 3 * n * 8, cudaMemcpyDeviceToHost, I.st));
-    CU(cudaStreamSynchronize(I.st));
-    double loss = 0.0;
-    for (size_t k = 0; k < 3 * n; k++) {
-        const double r = F[k] - fTarget[k];
-        loss += r * r;
-        w[k] = 2.0 * r;
+    B.gc = take(nc);
+    B.loss = take(parts);
+    // pinned staging for the target and the gradients (pageable copies of each array, with a synchronisation between the
+    // passes, took 0.5 ms of a 3.4 ms call at 8550 atoms)
+    if (I.hFmCap < std::max(3 * n, back)) {
+        if (I.hFm)
+            cudaFreeHost(I.hFm);
+        I.hFm = nullptr;
+        I.hFmCap = 0;
+        CU(cudaMallocHost((void**) &I.hFm, std::max(3 * n, back) * 8));
+        I.hFmCap = std::max(3 * n, back);
     }
-    CU(cudaMemcpyAsync(B.w, w.data(), 3 * n * 8, cudaMemcpyHostToDevice, I.st));
+    std::memcpy(I.hFm, fTarget, 3 * n * 8);
+    CU(cudaMemcpyAsync(B.w, I.hFm, 3 * n * 8, cudaMemcpyHostToDevice, I.st));
     const Dev d = I.makeDev(false, 0);
     const int tb = (int) ((n + 255) / 256);
-    std::vector<double> gqW(n), gRW(n), gcW(ncov), gqU(n), gRU(n), gaU(n), gcU(ncov);
-    auto fetch = [&](std::vector<double>& q_, std::vector<double>& R_, std::vector<double>* a_,
-                     std::vector<double>& c_) {
-        CU(cudaMemcpyAsync(q_.data(), B.gq, n * 8, cudaMemcpyDeviceToHost, I.st));
-        CU(cudaMemcpyAsync(R_.data(), B.gR, n * 8, cudaMemcpyDeviceToHost, I.st));
-        if (a_)
-            CU(cudaMemcpyAsync(a_->data(), B.ga, n * 8, cudaMemcpyDeviceToHost, I.st));
-        if (ncov)
-            CU(cudaMemcpyAsync(c_.data(), B.gc, ncov * 8, cudaMemcpyDeviceToHost, I.st));
-        CU(cudaStreamSynchronize(I.st));
-    };
+    k_fm_target<<<(int) parts, 256, 0, I.st>>>(d, B);
     // the pass along w (the final pass's fields and Hessian sums are still in place)
     k_fm_dp<<<tb, 256, 0, I.st>>>(d, B.w, B.dp);
     if (I.mixed())
@@ -2942,7 +2938,6 @@ double Engine::forceMatchingGrad(const double* fTarget, double tol, double* dq, 
         k_fm_cov<<<(int) ((ncov + 255) / 256), 256, 0, I.st>>>(d, B, 1);
     k_fm_rhs<<<(int) ((3 * n + 255) / 256), 256, 0, I.st>>>(d, B.Ed);
     CU(cudaGetLastError());
-    fetch(gqW, gRW, nullptr, gcW);
     // the adjoint solve: u in x
     const int its = I.solveDevice(tol);
     if (iterations)
@@ -2957,18 +2952,19 @@ double Engine::forceMatchingGrad(const double* fTarget, double tol, double* dq, 
     if (ncov)
         k_fm_cov<<<(int) ((ncov + 255) / 256), 256, 0, I.st>>>(d, B, 0);
     CU(cudaGetLastError());
-    fetch(gqU, gRU, &gaU, gcU);
-    for (size_t i = 0; i < n; i++) {
-        if (dq)
-            dq[i] = -gqW[i] + gqU[i];
-        if (dradius)
-            dradius[i] = -gRW[i] + gRU[i];
-        if (dalpha)
-            dalpha[i] = gaU[i];
-    }
+    CU(cudaMemcpyAsync(I.hFm, B.gq, back * 8, cudaMemcpyDeviceToHost, I.st));
+    CU(cudaStreamSynchronize(I.st));
+    if (dq)
+        std::memcpy(dq, I.hFm, n * 8);
+    if (dradius)
+        std::memcpy(dradius, I.hFm + n, n * 8);
+    if (dalpha)
+        std::memcpy(dalpha, I.hFm + 2 * n, n * 8);
     if (dstrength)
-        for (size_t m = 0; m < ncov; m++)
-            dstrength[m] = -gcW[m] + gcU[m];
+        std::memcpy(dstrength, I.hFm + 3 * n, ncov * 8);
+    double loss = 0.0;
+    for (size_t k = 0; k < parts; k++)
+        loss += I.hFm[3 * n + nc + k];
     return loss;
 }
 
