@@ -628,7 +628,12 @@ struct Engine::Impl {
             for (auto& g : groups)
                 fprintf(stderr, "pgm_b200 trace: FFT group %dx%dx%d, %d systems from %d, grid offset %lld, spectrum "
                         "offset %lld\n", g.K[0], g.K[1], g.K[2], g.count, g.first, g.gridOff, g.specOff);
-        convBlocks = std::max(1, std::min(512, (maxSpec + 255) / 256));
+        // (at least one per x-plane, so that the grid kernel's energy variant has a partial for each: at 20^3 the final
+        // pass otherwise takes cuFFT's chain, 20 us of a 320 us call)
+        int planes = 0;
+        for (int k = 0; k < nsys; k++)
+            planes = std::max(planes, sysK[k][0]);
+        convBlocks = std::max(std::min(planes, 512), std::min(512, (maxSpec + 255) / 256));
         // the field passes' transform pair with the influence product as one cluster kernel (a cluster per
         // system) when chosen (setTransforms, the autotuner) and every grid has at most FFT_MAXK points per
         // dimension with the prime factors 2, 3, 5 only; else cuFFT plans and the product kernel.  Cluster size:
