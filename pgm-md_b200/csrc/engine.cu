@@ -1384,8 +1384,8 @@ struct Engine::Impl {
     }
 
     // The whole CG solve after the permanent field (or for the right-hand side in b): one cooperative launch of the
-    // persistent kernel (one block per SM).
-    void launchPersistent(cudaStream_t sm, const Dev& d) {
+    // persistent kernel (one block per SM); finish: with the final pass's preparation and spread.
+    void launchPersistent(cudaStream_t sm, const Dev& d, bool finish = false) {
         PcgKernel kfn = pcgKernel(fftgKc);
         CU(cudaFuncSetAttribute((const void*) kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) pcgSmem));
         cudaLaunchConfig_t cfg = {};
@@ -1404,7 +1404,7 @@ struct Engine::Impl {
         const SysDev& S = sysHost[0];
         const double row = std::max(1.0, 4.0 / 3.0 * PI_D * S.cutoff * S.cutoff * S.cutoff * (n / S.volume));
         const int planeSlots = (int) std::min((double) n, PCG_PLANE_PAIRS / row);
-        CU(cudaLaunchKernelEx(&cfg, kfn, dp, planeSlots));
+        CU(cudaLaunchKernelEx(&cfg, kfn, dp, planeSlots, finish ? 1 : 0));
     }
 
     bool persistentMode() const { return tfMode == TF_PCG; }
@@ -1866,11 +1866,13 @@ struct Engine::Impl {
         CU(cudaGetLastError());
     }
 
-    template <typename R> void enqueuePost(cudaStream_t sm, cudaStream_t sd, const Dev& d) {
-        const int tb = (n + 255) / 256;
-        clearGrid<R>(sm, d);
-        k_final_prep<<<tb, 256, 0, sm>>>(d, s.polarizable ? 1 : 0);
-        launchSpread<R>(sm, d, 0, d.dtot);
+    // The final pass; prepared: the persistent kernel has done its preparation and spread.
+    template <typename R> void enqueuePost(cudaStream_t sm, cudaStream_t sd, const Dev& d, bool prepared = false) {
+        if (!prepared) {
+            clearGrid<R>(sm, d);
+            k_final_prep<<<(n + 255) / 256, 256, 0, sm>>>(d, s.polarizable ? 1 : 0);
+            launchSpread<R>(sm, d, 0, d.dtot);
+        }
         CU(cudaEventRecord(evFork, sm));
         CU(cudaStreamWaitEvent(sd, evFork, 0));
         // the final pass's transforms with the reciprocal energy: the grid kernel's energy variant where the field
@@ -1925,8 +1927,8 @@ struct Engine::Impl {
                 body = appendConditional(st, handle, cudaGraphCondTypeWhile);
             }
             else if (s.polarizable)
-                launchPersistent(st, d);
-            enqueuePost<R>(st, side, d);
+                launchPersistent(st, d, spreadFix());
+            enqueuePost<R>(st, side, d, s.polarizable && !loopNode && spreadFix());
         } catch (...) {
             capturing = false;
             cudaGraph_t g = nullptr;
@@ -1980,8 +1982,9 @@ struct Engine::Impl {
     template <typename R> void runDirect() {
         const Dev d = makeDev(false, 0);
         enqueuePre<R>(st, side, d);
-        if (s.polarizable && persistentMode()) {
-            launchPersistent(st, d);
+        const bool pcg = s.polarizable && persistentMode();
+        if (pcg) {
+            launchPersistent(st, d, spreadFix());
         } else if (s.polarizable) {
             static const bool trace = std::getenv("PGM_B200_TRACE") != nullptr;
             for (int it = 0; it <= s.maxIter + 1; it++) {
@@ -1999,7 +2002,7 @@ struct Engine::Impl {
                 enqueueIteration<R>(st, side, d);
             }
         }
-        enqueuePost<R>(st, side, d);
+        enqueuePost<R>(st, side, d, pcg && spreadFix());
     }
 
     // Mixed path with FP64 iterative refinement: the FP32-operator CG, then up to three rounds of
@@ -3044,8 +3047,9 @@ int Engine::kernelLaunches() const {
         it = std::max(it, (int) I.lastResults[(size_t) k * NRES + 14]);
     const int fp = 4, perIt = fp + (I.fusedGather() ? 1 : 2);
     const int pre = I.verletList() ? 7 + (I.lastBuilt ? 5 : 0) : 9;
-    const int solve = !I.s.polarizable ? 0 : I.persistentMode() ? fp + 1 : 2 * fp + 2 + perIt * it;
-    return pre + solve + 6 + (I.gvdwOn ? 1 : 0);
+    const bool pcg = I.s.polarizable && I.persistentMode();
+    const int solve = !I.s.polarizable ? 0 : pcg ? fp + 1 : 2 * fp + 2 + perIt * it;
+    return pre + solve + (pcg && I.spreadFix() ? 4 : 6) + (I.gvdwOn ? 1 : 0);
 }
 
 void Engine::kernelTimes(int reps, double* ms, void* flush, size_t flushBytes) {

@@ -13,7 +13,7 @@ typedef void (*GridKernel)(Dev, int);
 template <typename R> GridKernel gridKernel(int kc, bool energy);
 
 // The persistent CG kernel, compiled for the cubic grids of pcgSizes; any other grid (kc = 0) takes the general one.
-typedef void (*PcgKernel)(Dev, int);
+typedef void (*PcgKernel)(Dev, int, int);
 PcgKernel pcgKernel(int kc);
 
 }  // namespace pgmb200
