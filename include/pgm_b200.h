@@ -226,8 +226,10 @@ int pgm_engine_pair_lanes(pgm_engine* e);
  * with prime factors 2, 3, 5); 2 cuFFT 2D plans over the x-planes with one kernel for the x-lines and the
  * influence product (x extents up to 64 with prime factors 2, 3, 5); 3 one cooperative kernel per pass with a
  * thread block per x-plane of every system, the planes and the x-lines exchanged through L2 between two bounded
- * barriers (grids as for 1, every system's blocks resident together).  pgm_engine_transforms: the kind in use
- * (1, 2 and 3 only where the grids allow them). */
+ * barriers (grids as for 1, every system's blocks resident together); 4 that kernel for the passes around the CG solve
+ * and the whole solve as one persistent cooperative kernel (mixed precision, one system, order 6).  Until this call one
+ * system takes 4 where it applies, else 3 on the cubic grids that it is compiled for, else 0; batches 0.
+ * pgm_engine_transforms: the kind in use (1 to 4 only where the grids allow them). */
 int pgm_engine_set_transforms(pgm_engine* e, int mode);
 int pgm_engine_transforms(pgm_engine* e);
 

@@ -628,8 +628,8 @@ struct Engine::Impl {
             for (auto& g : groups)
                 fprintf(stderr, "pgm_b200 trace: FFT group %dx%dx%d, %d systems from %d, grid offset %lld, spectrum "
                         "offset %lld\n", g.K[0], g.K[1], g.K[2], g.count, g.first, g.gridOff, g.specOff);
-        // (at least one per x-plane, so that the grid kernel's energy variant has a partial for each: at 20^3 the final
-        // pass otherwise takes cuFFT's chain, 20 us of a 320 us call)
+        // (at least one per x-plane, so that the grid kernel's energy variant has a partial for each: a 20^3 grid's 17 sent
+        // the final pass through cuFFT's chain, four launches more)
         int planes = 0;
         for (int k = 0; k < nsys; k++)
             planes = std::max(planes, sysK[k][0]);

@@ -398,7 +398,9 @@ class Engine:
         """Field-pass transforms: 0 cuFFT 3D plans + influence product, 1 one cluster kernel per pass, 2 cuFFT 2D
         plans over the x-planes + one x-line kernel with the influence product, 3 one cooperative kernel with a
         block per x-plane, 4 that kernel for the field passes around the CG loop and the whole CG loop as one
-        persistent cooperative kernel (mixed precision, one system, order 6); transforms() tells which runs."""
+        persistent cooperative kernel (mixed precision, one system, order 6); transforms() tells which runs.  Until
+        this call one system takes 4 where it applies, else 3 on the cubic grids that it is compiled for, else 0, and a
+        batch 0."""
         _check(self._L.pgm_engine_set_transforms(self._h, int(mode)))
 
     def transforms(self):

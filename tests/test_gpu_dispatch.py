@@ -1,0 +1,81 @@
+"""The transforms that an engine takes until the caller chooses, and the persistent kernel at the edges of its slot split (fewer
+atoms than blocks, one slot a block, a remainder) and from each initial guess."""
+
+import numpy as np
+import pytest
+
+from conftest import PKG
+
+pytestmark = pytest.mark.gpu
+
+
+def engine(S, precision=1, tol=1e-8, zero_guess=False, order=6, predictor=0, **kw):
+    e = PKG.Engine(PKG.Settings(cutoff=S.cutoff, beta=S.beta, grid=S.grid, order=order, tol=tol, max_iter=500, peek=0.0,
+                                predictor=predictor, ke=PKG.systems.KE_DEFAULT, precision=precision,
+                                zero_guess=zero_guess, **kw))
+    e.set_system(S)
+    return e
+
+
+def water(molecules, K=None):
+    L = (molecules / 0.0334) ** (1 / 3)
+    K = K or max(8, PKG.systems.fft_size(L))
+    return PKG.systems.waters(molecules, L, seed=molecules, grid=(K, K, K), cutoff=min(9.0, L / 2), tol=1e-8)
+
+
+@pytest.mark.parametrize("molecules", [8, 49, 50, 99, 198, 443])   # 24, 147, 150, 297, 594, 1329 atoms on 148 blocks
+@pytest.mark.parametrize("zero_guess", [False, True])
+def test_persistent_kernel_slot_split(molecules, zero_guess):
+    """Against the graph loop with the grid kernel: the same iterations, and results that differ by the rounding of float
+    sums in another order (a few 2^-24 over sums whose terms cancel to a tenth: 3e-6)."""
+    S = water(molecules)
+    out = []
+    for mode in (3, 4):
+        e = engine(S, zero_guess=zero_guess)
+        e.set_transforms(mode)
+        assert e.transforms() == mode
+        r = e.compute(S.pos, S.box)
+        out.append((r.energy, r.forces, e.induced_dipoles(), r.iterations, r.strain))
+        x, _ = e.solve(out[-1][2], tol=1e-8)   # the adjoint's operator, from the zero guess
+        out[-1] += (x,)
+        e.close()
+    a, b = out
+    assert abs(a[3] - b[3]) <= 1
+    assert abs(a[0] - b[0]) <= 3e-6 * abs(a[0])
+    for k in (1, 2, 4, 5):
+        assert np.linalg.norm(a[k] - b[k]) <= 3e-6 * np.linalg.norm(a[k]), k
+
+
+def test_persistent_kernel_predicted_steps():
+    """Steps of a moving system, each guess of the predictor in turn (none, the last solution, mu3, mu4), with a kept list."""
+    S = water(120)
+    rng = np.random.default_rng(2)
+    phase = rng.uniform(0, 2 * np.pi, S.pos.shape)
+    traj = [S.pos + 0.005 * np.sin(2 * np.pi * t / 60 + phase) for t in range(7)]
+    runs = []
+    for mode in (3, 4):
+        e = engine(S, predictor=2, skin=0.1)
+        e.set_transforms(mode)
+        runs.append([e.compute(p, S.box) for p in traj])
+        e.close()
+    for a, b in zip(*runs):
+        assert abs(a.iterations - b.iterations) <= 1
+        assert abs(a.energy - b.energy) <= 3e-6 * abs(a.energy)
+        assert np.linalg.norm(a.forces - b.forces) <= 3e-6 * np.linalg.norm(a.forces)
+
+
+def test_transforms_without_a_choice():
+    S = water(64, K=16)
+    assert engine(S).transforms() == 4                       # mixed, one system, order 6
+    assert engine(S, precision=0).transforms() == 3          # FP64: the grid kernel
+    assert engine(S, order=5).transforms() == 3
+    assert engine(S, polarizable=False).transforms() == 3
+    assert engine(water(64, K=14)).transforms() == 0         # 14 = 2 x 7
+    e = engine(S)
+    e.set_pme_kernels(2)                                     # the caller's spread and gather run in the loop
+    assert e.transforms() == 3 and e.pme_kernels() == 2
+    e.set_transforms(0)                                      # the caller's choice stands
+    assert e.transforms() == 0
+    b = PKG.Engine(PKG.Settings(cutoff=S.cutoff, beta=S.beta, grid=S.grid, order=6, precision=1))
+    b.set_systems([S, S])
+    assert b.transforms() == 0                               # batches
