@@ -13,6 +13,7 @@
 #include "transforms.cuh"
 
 #include <algorithm>
+#include <array>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -507,7 +508,18 @@ struct Engine::Impl {
             covPartner.push_back(p[m]);
             covStrength.push_back(c[m]);
         }
+        const std::array<void*, 12> before = covalentBuffers();
         uploadCovalent();
+        if (exec && covalentBuffers() != before) {   // (more dipoles than before: the captured graph holds the old buffers)
+            cudaGraphExecDestroy(exec);
+            exec = nullptr;
+        }
+    }
+
+    std::array<void*, 12> covalentBuffers() const {
+        return {dCovAtom.p, dCovPartner.p, dCovStrength.p, dCovByAtomOff.p, dCovByAtom.p, dCovByPartnerOff.p,
+                dCovByPartner.p, dCovPartnerPos.p, dCovOwn.p, dCovOwnLen.p,
+                dCovOther.p, dCovOtherAtom.p};
     }
 
     void uploadCovalent() {

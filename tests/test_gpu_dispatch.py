@@ -79,3 +79,23 @@ def test_transforms_without_a_choice():
     b = PKG.Engine(PKG.Settings(cutoff=S.cutoff, beta=S.beta, grid=S.grid, order=6, precision=1))
     b.set_systems([S, S])
     assert b.transforms() == 0                               # batches
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_other_covalent_dipoles_after_an_evaluation(precision):
+    """A second set_covalent with fewer and then with more dipoles than the evaluation's graph was captured with gives what a
+    fresh engine gives (the same kernels on the same inputs: FP64 atomics aside, the same bits)."""
+    S = water(30)
+    half = len(S.cov_atom) // 2
+    e = PKG.Engine(PKG.Settings(cutoff=S.cutoff, beta=S.beta, grid=S.grid, order=6, tol=1e-8, max_iter=500, peek=0.0,
+                                predictor=0, ke=PKG.systems.KE_DEFAULT, precision=precision, skin=0.0))
+    e.set_atoms(S.q, S.radius, S.alpha)
+    for m in (half, 2, len(S.cov_atom)):
+        e.set_covalent(S.cov_atom[:m], S.cov_partner[:m], S.cov_strength[:m])
+        for _ in range(2):
+            r = e.compute(S.pos, S.box)
+        fresh = engine(S, precision=precision, skin=0.0)
+        fresh.set_covalent(S.cov_atom[:m], S.cov_partner[:m], S.cov_strength[:m])
+        f = fresh.compute(S.pos, S.box)
+        assert abs(r.energy - f.energy) <= 1e-12 * abs(f.energy)
+        assert np.linalg.norm(r.forces - f.forces) <= 1e-12 * np.linalg.norm(f.forces)
