@@ -1244,9 +1244,11 @@ struct Engine::Impl {
         const int* K = sysK[0].data();
         pcgBlocks = std::min(sms, PCG_MAX_BLOCKS);   // (one per SM; the plane blocks are 0 .. K0-1)
         pcgSmem = pcgSmemBytes((n + pcgBlocks - 1) / pcgBlocks, fftgBuf);
-        if (!coop || pcgSmem > (size_t) optin || K[0] + PCG_MIN_PAIR_BLOCKS > pcgBlocks)
-            return;
         PcgKernel kfn = pcgKernel(fftgKc);
+        cudaFuncAttributes fa;   // (a block's static shared memory counts against the limit too)
+        CU(cudaFuncGetAttributes(&fa, (const void*) kfn));
+        if (!coop || pcgSmem + fa.sharedSizeBytes > (size_t) optin || K[0] + PCG_MIN_PAIR_BLOCKS > pcgBlocks)
+            return;
         CU(cudaFuncSetAttribute((const void*) kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) pcgSmem));
         int perSm = 0;
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kfn, PCG_THREADS, pcgSmem));
