@@ -1180,11 +1180,26 @@ struct Engine::Impl {
         }
     }
 
+    // Whether a block of kernel f can have `bytes` of dynamic shared memory beside its static part on this GPU; allows it all
+    // that there is.  The attribute belongs to the function, not to an engine: set to one engine's size it would refuse the
+    // launches of another that needs more of the same instance, so every engine sets the same value, and none at a launch.
+    static bool allowSharedMemory(const void* f, size_t bytes) {
+        int dev = 0, optin = 0;
+        CU(cudaGetDevice(&dev));
+        CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        cudaFuncAttributes fa;
+        CU(cudaFuncGetAttributes(&fa, f));
+        const size_t most = (size_t) optin - fa.sharedSizeBytes;
+        CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) most));
+        return bytes <= most;
+    }
+
     // Attributes of the cluster transform kernel; false when no cluster of its size fits on this GPU.
     template <typename R> bool prepareCluster() {
         const void* f = (const void*) k_fft_cluster<R>;
         CU(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fftcSmem));
+        if (!allowSharedMemory(f, fftcSmem))
+            return false;
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1207,20 +1222,16 @@ struct Engine::Impl {
     // Attributes of the grid-transform kernel; false when its blocks (a block per x-plane of every system) cannot
     // all be resident at once on this GPU or a block's shared memory does not fit.
     template <typename R> bool prepareGrid() {
-        int optin = 0, sms = 0, coop = 0;
-        CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, devId));
+        int sms = 0, coop = 0;
         CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devId));
         CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, devId));
-        if (!coop || fftgSmem > (size_t) optin)
+        if (!coop || !allowSharedMemory((const void*) gridKernel<R>(fftgKc, false), fftgSmem) ||
+            !allowSharedMemory((const void*) gridKernel<R>(fftgKc, true), fftgSmem))
             return false;
-        CU(cudaFuncSetAttribute((const void*) gridKernel<R>(fftgKc, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int) fftgSmem));
         int perSm = 0;
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, gridKernel<R>(fftgKc, false), FftgThreads<R>::n,
                                                          fftgSmem));
         // the final pass's variant: every block resident too, and a conv partial of its own for each x-plane
-        CU(cudaFuncSetAttribute((const void*) gridKernel<R>(fftgKc, true),
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fftgSmem));
         int perSmE = 0;
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSmE, gridKernel<R>(fftgKc, true), FftgThreads<R>::n,
                                                          fftgSmem));
@@ -1237,19 +1248,15 @@ struct Engine::Impl {
         pcgOk = false;
         if (!mixed() || nsys != 1 || !gridOk || s.order != 6 || !s.polarizable)
             return;
-        int sms = 0, coop = 0, optin = 0;
+        int sms = 0, coop = 0;
         CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devId));
         CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, devId));
-        CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, devId));
         const int* K = sysK[0].data();
         pcgBlocks = std::min(sms, PCG_MAX_BLOCKS);   // (one per SM; the plane blocks are 0 .. K0-1)
         pcgSmem = pcgSmemBytes((n + pcgBlocks - 1) / pcgBlocks, fftgBuf);
         PcgKernel kfn = pcgKernel(fftgKc);
-        cudaFuncAttributes fa;   // (a block's static shared memory counts against the limit too)
-        CU(cudaFuncGetAttributes(&fa, (const void*) kfn));
-        if (!coop || pcgSmem + fa.sharedSizeBytes > (size_t) optin || K[0] + PCG_MIN_PAIR_BLOCKS > pcgBlocks)
+        if (!coop || K[0] + PCG_MIN_PAIR_BLOCKS > pcgBlocks || !allowSharedMemory((const void*) kfn, pcgSmem))
             return;
-        CU(cudaFuncSetAttribute((const void*) kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) pcgSmem));
         int perSm = 0;
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kfn, PCG_THREADS, pcgSmem));
         if (perSm < 1)
@@ -1267,19 +1274,15 @@ struct Engine::Impl {
         const int* K = sysK[0].data();
         planeNyc = (K[1] + PL_YCH - 1) / PL_YCH;
         planeSmem = (size_t) (PL_YCH + 5) * K[2] * sizeof(float);
-        int optin = 0;
-        CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, devId));
-        if (planeSmem > (size_t) optin)
+        if (!allowSharedMemory((const void*) k_spread_planes<6>, planeSmem) ||
+            !allowSharedMemory((const void*) k_gather_planes<6>, planeSmem))
             return;
-        for (const void* f : {(const void*) k_spread_planes<6>, (const void*) k_gather_planes<6>})
-            CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) planeSmem));
         const size_t nbins = (size_t) K[0] * planeNyc;
         if (nbins > (size_t) PL_MAX_SMEM_BINS)
             return;   // (the binning kernels keep a block's histogram of every bin in shared memory)
-        CU(cudaFuncSetAttribute((const void*) k_plane_bin_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int) (nbins * sizeof(int))));
-        CU(cudaFuncSetAttribute((const void*) k_plane_bin_fill<6>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int) (2 * nbins * sizeof(int))));
+        if (!allowSharedMemory((const void*) k_plane_bin_count, nbins * sizeof(int)) ||
+            !allowSharedMemory((const void*) k_plane_bin_fill<6>, 2 * nbins * sizeof(int)))
+            return;
         dPmeRec.ensure((size_t) n * sizeof(PmeRec<6>));
         dPmeBins.ensure((std::max<size_t>(nbins, FFT_MAXK) + 1) * sizeof(int));
         dBinCount.ensure(nbins * sizeof(int));
@@ -1401,7 +1404,6 @@ struct Engine::Impl {
     // persistent kernel (one block per SM); finish: with the final pass's preparation and spread.
     void launchPersistent(cudaStream_t sm, const Dev& d, bool finish = false) {
         PcgKernel kfn = pcgKernel(fftgKc);
-        CU(cudaFuncSetAttribute((const void*) kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) pcgSmem));
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeCooperative;
