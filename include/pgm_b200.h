@@ -88,7 +88,8 @@ int pgm_engine_set_candidates(pgm_engine* e, int nseg, const int* seg_i, const i
                               const int* cand_j);
 /* Self-test of the failure path of the grid transforms' barriers (no counterpart in the reference): one block
  * waits at a barrier that expects two; the wait gives up after its bounded number of polls, sets the error flag
- * and returns.  *flag = 1 when it did (the expected outcome), *seconds the device time of the launch. */
+ * and returns.  *flag = 1 when it did (the expected outcome), *seconds the device time of the launch.  After an
+ * evaluation by the grid kernel (transforms 3 or 4): and when later launches that find the flag return without waiting. */
 int pgm_engine_probe_barrier_timeout(pgm_engine* e, int* flag, double* seconds);
 /* The coefficients c[0..k-1] (k <= 32) of the GVDW dispersion's G(y)/G(0) = sum c_m y^(2m) that set_gvdw uses
  * below y = 0.6, derived from the series of erf and exp (no counterpart in the reference, which tabulates them in

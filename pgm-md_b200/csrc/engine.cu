@@ -2294,14 +2294,16 @@ void Engine::setAtoms(int n, const double* q, const double* radius, const double
 
 // Self-test of the grid transforms' bounded barrier: one block waits at a barrier that expects two; the wait
 // runs out, sets the error flag and returns.  Returns the flag (1: the wait gave up as designed) and the
-// device time of the launch.
+// device time of the launch.  After an evaluation by the grid kernel, launches of it with that flag follow, on the
+// probe's barrier words: they return without a barrier (else 0 is returned).
 int Engine::probeBarrierTimeout(double* seconds) {
     Impl& I = *impl;
     I.selectDevice();
     void* mem = nullptr;
-    CU(cudaMalloc(&mem, 64 * sizeof(int)));
+    const size_t count = 32 + 2 * (size_t) I.nsys;   // the flags, the probe's barrier, the grid kernel's barriers
+    CU(cudaMalloc(&mem, count * sizeof(int)));
     int* words = (int*) mem;
-    CU(cudaMemsetAsync(words, 0, 64 * sizeof(int), I.st));
+    CU(cudaMemsetAsync(words, 0, count * sizeof(int), I.st));
     cudaEvent_t a, b;
     CU(cudaEventCreate(&a));
     CU(cudaEventCreate(&b));
@@ -2309,8 +2311,18 @@ int Engine::probeBarrierTimeout(double* seconds) {
     k_barrier_probe<<<1, 32, 0, I.st>>>((unsigned*) (words + 16), words);
     CU(cudaGetLastError());
     CU(cudaEventRecord(b, I.st));
-    int flags[16];
-    CU(cudaMemcpyAsync(flags, words, sizeof(flags), cudaMemcpyDeviceToHost, I.st));
+    if (I.haveResult && (I.tfMode == Impl::TF_GRID || I.tfMode == Impl::TF_PCG)) {
+        Dev d = I.makeDev(false, 0);
+        d.flags = words;
+        d.fftgBar = (unsigned*) (words + 32);
+        for (int k = 0; k < 2; k++)
+            if (I.mixed())
+                I.launchGrid<float>(I.st, d, 0, false);
+            else
+                I.launchGrid<double>(I.st, d, 0, false);
+    }
+    std::vector<int> flags(count);
+    CU(cudaMemcpyAsync(flags.data(), words, count * sizeof(int), cudaMemcpyDeviceToHost, I.st));
     CU(cudaStreamSynchronize(I.st));
     float ms = 0.0f;
     CU(cudaEventElapsedTime(&ms, a, b));
@@ -2319,6 +2331,9 @@ int Engine::probeBarrierTimeout(double* seconds) {
     CU(cudaFree(mem));
     if (seconds)
         *seconds = ms * 1e-3;
+    for (size_t k = 32; k < count; k++)
+        if (flags[k] != 0)
+            return 0;
     return flags[11];
 }
 

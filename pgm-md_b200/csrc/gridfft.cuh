@@ -91,7 +91,10 @@ __global__ void __launch_bounds__(FftgThreads<R>::n, FftgThreads<R>::perSm) k_ff
         W1[m] = tw[S.twOff[1] + m];
     for (int m = tid; m < K2; m += nT)
         W2[m] = tw[S.twOff[2] + m];
-    __syncthreads();
+    // A barrier of an earlier launch of this call gave up: its counter is out of step, so every wait here would run out too,
+    // a second each in every iteration still enqueued.  The results are undefined already; the host reports the flag.
+    if (__syncthreads_or(tid == 0 && dv.flags[11] != 0))
+        return;
     const PlaneFft<R, KC> fft(K0, K1, K2, b0, b1, W0, W1, W2);
     const int nline = fft.nline, l0 = x * fft.lpb, nl = min(nline, l0 + fft.lpb) - l0;
     R* const gx = (R*) dv.grid + S.gridOff + (size_t) x * K1 * K2;
