@@ -2174,20 +2174,25 @@ struct Engine::Impl {
     size_t flagBytes() const { return (16 + 2 * (size_t) nsys + 2) * sizeof(int); }
 
     // After the flags came back: a grid-transform barrier that gave up leaves the evaluation's results
-    // undefined (the barrier words are reset at the next evaluation's start).
-    void barrierCheck() const {
-        if (hFlags[11])
-            throw std::runtime_error("pgm_b200: a grid-transform barrier gave up waiting (blocks not resident "
-                                     "together?)");
+    // undefined (the barrier words are reset at the next evaluation's start) and sources in the fixed-point grids, which
+    // every spread adds to and only a conversion clears: the next evaluation would add to them.
+    void barrierCheck() {
+        if (!hFlags[11])
+            return;
+        for (Buf* b : {&dGridFix, &dGridFix2})
+            if (b->p)
+                CU(cudaMemsetAsync(b->p, 0, gridTotal * 8, st));
+        throw std::runtime_error("pgm_b200: a grid-transform barrier gave up waiting (blocks not resident "
+                                 "together?)");
     }
 
     // Waits for the launched evaluation; false if it must be repeated (pair-list capacity grown).
     bool finish() {
         CU(cudaEventSynchronize(evDone));
         launched = false;
+        barrierCheck();
         if (hFlags[1])
             throw std::runtime_error("pgm_b200: pair image shift beyond 3 boxes (positions far outside the box?)");
-        barrierCheck();
         lastBuilt = hFlags[8] != 0;
         if (hFlags[8]) {
             builds++;
@@ -2294,8 +2299,9 @@ void Engine::setAtoms(int n, const double* q, const double* radius, const double
 
 // Self-test of the grid transforms' bounded barrier: one block waits at a barrier that expects two; the wait
 // runs out, sets the error flag and returns.  Returns the flag (1: the wait gave up as designed) and the
-// device time of the launch.  After an evaluation by the grid kernel, launches of it with that flag follow, on the
-// probe's barrier words: they return without a barrier (else 0 is returned).
+// device time of the launch.  After an evaluation by the grid kernel, a spread and launches of that kernel
+// with that flag follow, on the probe's barrier words: they return without a barrier (else 0 is returned).  The engine is
+// left as a call is left whose barrier gave up, by the same host path.
 int Engine::probeBarrierTimeout(double* seconds) {
     Impl& I = *impl;
     I.selectDevice();
@@ -2315,9 +2321,11 @@ int Engine::probeBarrierTimeout(double* seconds) {
         Dev d = I.makeDev(false, 0);
         d.flags = words;
         d.fftgBar = (unsigned*) (words + 32);
+        if (I.mixed())
+            I.launchSpread<float>(I.st, d, 1, d.x);
         for (int k = 0; k < 2; k++)
             if (I.mixed())
-                I.launchGrid<float>(I.st, d, 0, false);
+                I.launchGrid<float>(I.st, d, d.gridFix ? 2 : 0, false);
             else
                 I.launchGrid<double>(I.st, d, 0, false);
     }
@@ -2331,6 +2339,11 @@ int Engine::probeBarrierTimeout(double* seconds) {
     CU(cudaFree(mem));
     if (seconds)
         *seconds = ms * 1e-3;
+    std::copy(flags.begin(), flags.begin() + 16, I.hFlags);
+    try {
+        I.barrierCheck();
+    } catch (const std::runtime_error&) {   // (that the wait gave up: what this call returns)
+    }
     for (size_t k = 32; k < count; k++)
         if (flags[k] != 0)
             return 0;

@@ -28,7 +28,7 @@ def test_grid_barrier_wait_gives_up_and_reports():
                                                  (0, 3, (18, 20, 24))])
 def test_launches_after_a_barrier_gave_up_do_not_wait(precision, mode, grid):
     """Grid-kernel launches that find the error flag set return at once, in place of a second at each of their barriers; the
-    next evaluation is unchanged."""
+    next evaluation is unchanged (the sources that the self-test's spread left on the fixed-point grid are gone)."""
     S = PKG.systems.water216()
     eng = PKG.Engine(PKG.Settings(cutoff=S.cutoff, beta=S.beta, grid=grid, order=S.order, tol=1e-8, predictor=0,
                                   precision=precision))
