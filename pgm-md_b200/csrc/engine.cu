@@ -1455,19 +1455,26 @@ struct Engine::Impl {
                      const double* quadD, int withQ);
 
     // The transform mode in use: the caller's choice where the systems' grids allow it, else cuFFT.  Until the caller
-    // chooses, one system takes the persistent kernel (with its own spread and gather, so not when the caller chose
-    // other PME kernels or the dual first pass), else the grid kernel where it is compiled for the grid.  Measured on one
-    // B200, us an evaluation, persistent / grid kernel / cuFFT: mixed 72 atoms (9^3) 252 / 384 / 357, 648 (20^3) 285 / 422
-    // / 417, 4113 (36^3) 420 / 562 / 562, 8550 (48^3) 593 / 717 / 929, 12288 (50^3) 705 / 917 / 877; FP64 93 (48^3) - / 364
-    // / 447, 8550 (48^3) - / 945 / 1039, but 648 (20^3, the general grid kernel) - / 423 / 410.  Batches keep cuFFT, whose plans
-    // take all systems of a shape at once.
+    // chooses, one system on a grid that the kernels are compiled for (fftgKc: cubic) takes the persistent kernel, with its
+    // own spread and gather, so not when the caller chose other PME kernels or the dual first pass, else the grid kernel.
+    // Measured on one B200, us an evaluation, persistent / grid kernel / cuFFT (mode 4 / 3 / 0), the lines of the rule:
+    //   cubic, mixed: 72 atoms (9^3) 252 / 384 / 357, 648 (20^3) 275 / 346 / 411, 2700 (30^3) 310 / 375 / 501, 8550 (48^3)
+    //     593 / 717 / 929, 15777 (54^3) 817 / 943 / 1044, 26244 (64^3) 1075 / 1246 / 1361
+    //   other grids, mixed: 60 atoms (6^3) 421 / 327 / 300, 2700 (24 x 30 x 36) 630 / 462 / 489, 10410 (40 x 48 x 54) 1063 /
+    //     831 / 821, 15777 (48 x 54 x 60) 1237 / 1067 / 1038; FP64 648 (18 x 20 x 24) - / 424 / 415, 15777 - / 1191 / 1189: the
+    //     general instances' run-time radices, cuFFT stays
+    //   PCG_RULE_SMEM, mixed: 85500 atoms (64^3, 193 KB) 3062 / 3199 / 3321, 87000 (196 KB) 3453 / 3259 / 3363; 93000 (48^3,
+    //     193 KB) 3185 / 3544 / 3621, 98304 (203 KB) 3743 / 3670 / 3779
+    //   FP64: 4113 (36^3) - / 493 / 547, 8550 (48^3) - / 935 / 1021, 39000 (60^3) - / 2362 / 2398; 64^3, whose passes take two
+    //     rounds of the block's 256 threads: 9000 atoms - / 802 / 850, 15900 - / 1229 / 1210, 26244 - / 1757 / 1711
+    // Batches keep cuFFT, whose plans take all systems of a shape at once.
     void selectTransforms() {
         int m = TF_CUFFT;
-        if (tfWant == TF_AUTO && nsys == 1) {
+        if (tfWant == TF_AUTO && nsys == 1 && gridOk && fftgKc > 0) {
             const char* dual = std::getenv("PGM_B200_DUAL");
-            if (pcgOk && pmeWant == 0 && !(dual && dual[0] == '1'))
+            if (pcgOk && pcgSmem <= PCG_RULE_SMEM && pmeWant == 0 && !(dual && dual[0] == '1'))
                 m = TF_PCG;
-            else if (gridOk && fftgKc > 0)
+            else if (mixed() || fftgKc < 64 || n <= 12000)
                 m = TF_GRID;
         }
         if (tfWant == TF_CLUSTER && clusterOk)

@@ -42,6 +42,10 @@ constexpr int PCG_THREADS = 1024;
 constexpr int PCG_MAX_BLOCKS = 160;          // the totals' loads are unrolled for at most this many blocks
 constexpr int PCG_MIN_PAIR_BLOCKS = 16;      // blocks left for the pair pass beside the plane blocks
 constexpr int PCG_SLOT_LANES = 16;           // lanes per slot in the spread and gather phases
+// The rule (selectTransforms) takes the kernel up to this much dynamic shared memory a block: with its static part and the
+// 1 KB that the system keeps it still fits the 196 KB split of an SM, and the pair pass has 60 KB of L1; beyond, the split is
+// 228 KB and the gathers of the pair pass miss (an evaluation of 85500 atoms at 64^3 takes 3062 us, of 87000 3453).
+constexpr size_t PCG_RULE_SMEM = 198000;
 // Directed pairs that a block sums while a plane block transforms its plane (9.9 us at 48^3): the plane blocks take
 // that many fewer of the pair pass's rows, if any.
 constexpr int PCG_PLANE_PAIRS = 32000;

@@ -107,8 +107,8 @@ public:
     // field-pass transforms: 0 cuFFT 3D plans + influence product kernel, 1 one cluster kernel per launch,
     // 2 cuFFT 2D plans over the x-planes + one x-line kernel with the influence product, 3 one cooperative kernel
     // with a block per x-plane, 4 that kernel around the CG solve and the solve as one persistent kernel (1 to 4 where
-    // the grids allow them; transforms() tells which runs).  Until the caller chooses: one system 4, else 3 on the grids
-    // it is compiled for, else 0; batches 0
+    // the grids allow them; transforms() tells which runs).  Until the caller chooses: one system on a cubic grid that
+    // they are compiled for 4, else 3, by the rule of selectTransforms; any other grid and batches 0
     void setTransforms(int mode);
     // PME spread / gather of the field passes: 0 a warp per atom, 1 plane-owner tiles in shared memory (mixed
     // precision, one system, order 6), 2 float4 lines (mixed precision, orders 4, 5, 6, 8), 3 cell-group tiles

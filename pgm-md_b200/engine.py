@@ -399,8 +399,9 @@ class Engine:
         plans over the x-planes + one x-line kernel with the influence product, 3 one cooperative kernel with a
         block per x-plane, 4 that kernel for the field passes around the CG loop and the whole CG loop as one
         persistent cooperative kernel (mixed precision, one system, order 6); transforms() tells which runs.  Until
-        this call one system takes 4 where it applies, else 3 on the cubic grids that it is compiled for, else 0, and a
-        batch 0."""
+        this call one system on a cubic grid (8 to 64 points, prime factors 2, 3, 5) takes 4 where it applies (up to 85000
+        to 100000 atoms by grid), else 3 (in FP64 at 64 points up to 12000 atoms), any other grid and a batch 0; the
+        choice stands for the engine's life."""
         _check(self._L.pgm_engine_set_transforms(self._h, int(mode)))
 
     def transforms(self):

@@ -82,6 +82,28 @@ def test_transforms_without_a_choice():
 
 
 @pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("grid", [(6, 6, 6), (10, 12, 15), (24, 30, 36), (16, 16, 20)])
+def test_grids_without_an_instance_keep_cufft(grid, precision):
+    """The general instances of the persistent and the grid kernel are slower than cuFFT: only a choice takes them."""
+    S = PKG.systems.waters(20, 9.0, seed=3, grid=grid, cutoff=4.4, tol=1e-6)
+    e = engine(S, precision=precision)
+    assert e.transforms() == 0
+    for mode in (3, 4):
+        e.set_transforms(mode)
+        assert e.transforms() == (mode if mode == 3 or precision == 1 else 0)
+    e.close()
+
+
+@pytest.mark.parametrize("atoms,K,precision,mode", [(85500, 64, 1, 4), (87000, 64, 1, 3), (93000, 48, 1, 4), (98304, 48, 1, 3),
+                                                    (12000, 64, 0, 3), (12300, 64, 0, 0), (39000, 60, 0, 3)])
+def test_atom_counts_of_the_rule(atoms, K, precision, mode):
+    e = PKG.Engine(PKG.Settings(cutoff=0.9, beta=3.5, grid=(K, K, K), order=6, precision=precision))
+    e.set_atoms(np.zeros(atoms), np.full(atoms, 0.07), np.full(atoms, 1e-3))
+    assert e.transforms() == mode
+    e.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
 def test_other_covalent_dipoles_after_an_evaluation(precision):
     """A second set_covalent with fewer and then with more dipoles than the evaluation's graph was captured with gives what a
     fresh engine gives (the same kernels on the same inputs: FP64 atomics aside, the same bits)."""
