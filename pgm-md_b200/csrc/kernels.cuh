@@ -558,11 +558,11 @@ __global__ void k_list_from_candidates(Dev dv) {
 template <typename R> struct PairRec { static constexpr bool storeX = false; };
 template <> struct PairRec<float> { static constexpr bool storeX = true; };
 
-// x = pw_i - pw_j - w.H of the list entry e in double, rounded to R (most pairs are inside the box: w = 0).  For the record
-// passes; in the FP64 field and final passes the branch keeps the loads of an unrolled round apart (22.6 -> 24.6 us and
-// 42 -> 59 us at 8550 atoms).
-template <typename R>
-__device__ __forceinline__ void pairVector(double4 pwj, double4 pwi, uint32_t e, const double* H, R* x) {
+// x = pw_i - pw_j - w.H of the list entry e (most pairs are inside the box: w = 0).  For the compaction, which tests many
+// more pairs than it keeps (list + compaction at 8550 / 12288 atoms, us: mixed 149.5 -> 144.2 / 214.3 -> 209.1, FP64 176.9 ->
+// 175.3 / 243.8 -> 241.0).  Elsewhere the branch keeps the loads of an unrolled round apart: list + records without a skin of
+// 64 boxes of 200 waters 349 -> 361 mixed, 500 -> 504 FP64, the FP64 field pass 22.6 -> 24.6, the final pass 42 -> 59.
+__device__ __forceinline__ void pairVector(double4 pwj, double4 pwi, uint32_t e, const double* H, double* x) {
     double x0 = pwi.x - pwj.x, x1 = pwi.y - pwj.y, x2 = pwi.z - pwj.z;
     if ((int) (e >> 23) != NO_SHIFT) {
         double sh[3];
@@ -571,9 +571,9 @@ __device__ __forceinline__ void pairVector(double4 pwj, double4 pwi, uint32_t e,
         x1 -= sh[1];
         x2 -= sh[2];
     }
-    x[0] = (R) x0;
-    x[1] = (R) x1;
-    x[2] = (R) x2;
+    x[0] = x0;
+    x[1] = x1;
+    x[2] = x2;
 }
 
 // The pair records of every listed pair (the list of the evaluation) in precision R with G0..G3 by
@@ -604,10 +604,12 @@ __global__ void __launch_bounds__(256) k_pair_kernels(Dev dv) {
     for (int t = lane; t < cnt; t += 32) {
         const uint32_t e = row[t];
         const int js = entrySlot(e);
-        R xr[3];
-        pairVector(dv.posS[js], pwi, e, S.H, xr);
+        double sh[3];
+        entryShift(e, S.H, sh);
+        const double4 pwj = dv.posS[js];
+        const double x0 = pwi.x - pwj.x - sh[0], x1 = pwi.y - pwj.y - sh[1], x2 = pwi.z - pwj.z - sh[2];
         const R Rj = (R) dv.radS[js], Rr = (R) Ri;
-        const R xr0 = xr[0], xr1 = xr[1], xr2 = xr[2];
+        const R xr0 = (R) x0, xr1 = (R) x1, xr2 = (R) x2;
         const R r = fsqrt(xr0 * xr0 + xr1 * xr1 + xr2 * xr2);
         const R a = R(1) / fsqrt(R(2) * (Rr * Rr + Rj * Rj));
         R G[4];
