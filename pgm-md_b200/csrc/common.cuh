@@ -200,6 +200,7 @@ struct Dev {
     float4* srcW;
     float4* gpart;
     double* pcgPartial;
+    unsigned char* pcgState;  // the persistent kernel's per-slot state where shared memory does not hold it
     unsigned* pcgBar;
     // graph
     int loopCond;                          // 1: the CG loop is a conditional while node (k_cg_init sets it)

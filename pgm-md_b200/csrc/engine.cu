@@ -199,6 +199,7 @@ struct Engine::Impl {
     size_t planeSmem = 0;
     int pcgBlocks = 0;         // its blocks (one per SM)
     size_t pcgSmem = 0;
+    bool pcgShared = true;     // its slots' state in shared memory (else in dPcgState)
     int fftcBuf = 0, fftcC = 16, fftgBuf = 0, maxK0 = 0;
     int fftgKc = 0;            // the grid transforms' compile-time size (every grid fftgKc^3), or 0
     size_t fftgSmem = 0;
@@ -210,7 +211,7 @@ struct Engine::Impl {
     Buf dSys, dAtomSys, dQ, dR, dAlpha, dPosIn, dWrap, dCellOf, dCellRank, dBase, dFr, dCellCount, dCellStart,
         dSlotAtom, dSlotTmp, dPosS, dOrigS, dWrapS, dSpl, dBaseS, dRadS, dList, dListCount, dPairA, dPairB, dPairC, dFlags, dDS, dPerm, dMu, dDtot, dB, dX, dRv, dZ, dP, dAp,
         dDS2, dEpair2, dErec2, dGrid2, dGridFix, dGridFix2,
-        dScal, dPartial, dGPartial, dHrec, dFm, dPmeRec, dPmeBins, dSrcW, dGPart, dPcgPartial, dBinCount, dActive, dActSys, dSysCounter, dEpair, dErec, dFpair, dSpair, dFrec, dEtot, dFin, dPot, dForces, dResults,
+        dScal, dPartial, dGPartial, dHrec, dFm, dPmeRec, dPmeBins, dSrcW, dGPart, dPcgPartial, dPcgState, dBinCount, dActive, dActSys, dSysCounter, dEpair, dErec, dFpair, dSpair, dFrec, dEtot, dFin, dPot, dForces, dResults,
         dConvPartial, dConvOff, dGrid, dSpec, dInfl, dTwiddle, dModuli, dCovAtom, dCovPartner, dCovStrength, dCovByAtomOff,
         dCovByAtom, dCovByPartnerOff, dCovByPartner, dCovPartnerPos, dCovOwn, dCovOwnLen, dCovOther, dCovOtherAtom, dChunkSys, dChunkBegin, dChunkEnd, dHist, dGlobal, dCtl,
         dGradQ, dGradR, dSList, dSListCount, dPosBuild, dAtomSlot, dCandStart, dCandJ, dCandT, dGv, dSkipStart, dSkipJ;
@@ -306,7 +307,7 @@ struct Engine::Impl {
                       &dCellCount, &dCellStart, &dSlotAtom, &dSlotTmp, &dPosS, &dOrigS, &dWrapS, &dSpl, &dBaseS, &dRadS, &dList, &dListCount, &dPairA, &dPairB, &dPairC, &dFlags, &dDS,
                       &dDS2, &dEpair2, &dErec2, &dGrid2, &dGridFix, &dGridFix2,
                       &dPerm, &dMu, &dDtot, &dB, &dX, &dRv, &dZ, &dP, &dAp, &dScal, &dPartial, &dGPartial, &dHrec, &dFm, &dPmeRec, &dPmeBins, &dSrcW, &dGPart,
-                      &dPcgPartial, &dBinCount, &dActive, &dActSys, &dSysCounter, &dEpair,
+                      &dPcgPartial, &dPcgState, &dBinCount, &dActive, &dActSys, &dSysCounter, &dEpair,
                       &dErec, &dFpair, &dSpair, &dFrec, &dEtot, &dFin, &dPot, &dForces, &dResults, &dConvPartial,
                       &dConvOff, &dGrid, &dSpec, &dInfl, &dTwiddle, &dModuli, &dCovAtom, &dCovPartner, &dCovStrength,
                       &dCovByAtomOff, &dCovByAtom, &dCovByPartnerOff, &dCovByPartner, &dCovPartnerPos, &dCovOwn,
@@ -1116,6 +1117,7 @@ struct Engine::Impl {
         d.srcW = dSrcW.as<float4>();
         d.gpart = dGPart.as<float4>();
         d.pcgPartial = dPcgPartial.as<double>();
+        d.pcgState = dPcgState.as<unsigned char>();
         d.moduli = dModuli.as<double>();
         d.ncov = (int) covAtom.size();
         d.covAtom = dCovAtom.as<int>();
@@ -1253,10 +1255,16 @@ struct Engine::Impl {
         CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, devId));
         const int* K = sysK[0].data();
         pcgBlocks = std::min(sms, PCG_MAX_BLOCKS);   // (one per SM; the plane blocks are 0 .. K0-1)
-        pcgSmem = pcgSmemBytes((n + pcgBlocks - 1) / pcgBlocks, fftgBuf);
-        PcgKernel kfn = pcgKernel(fftgKc);
-        if (!coop || K[0] + PCG_MIN_PAIR_BLOCKS > pcgBlocks || !allowSharedMemory((const void*) kfn, pcgSmem))
+        if (!coop || K[0] + PCG_MIN_PAIR_BLOCKS > pcgBlocks)
             return;
+        pcgSmem = pcgTransformBytes(fftgBuf) + pcgStateBytes((n + pcgBlocks - 1) / pcgBlocks);
+        pcgShared = allowSharedMemory((const void*) pcgKernel(fftgKc, true), pcgSmem);
+        if (!pcgShared) {   // (more than about 100000 atoms)
+            pcgSmem = pcgTransformBytes(fftgBuf);
+            if (!allowSharedMemory((const void*) pcgKernel(fftgKc, false), pcgSmem))
+                return;
+        }
+        PcgKernel kfn = pcgKernel(fftgKc, pcgShared);
         int perSm = 0;
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kfn, PCG_THREADS, pcgSmem));
         if (perSm < 1)
@@ -1403,7 +1411,7 @@ struct Engine::Impl {
     // The whole CG solve after the permanent field (or for the right-hand side in b): one cooperative launch of the
     // persistent kernel (one block per SM); finish: with the final pass's preparation and spread.
     void launchPersistent(cudaStream_t sm, const Dev& d, bool finish = false) {
-        PcgKernel kfn = pcgKernel(fftgKc);
+        PcgKernel kfn = pcgKernel(fftgKc, pcgShared);
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeCooperative;
@@ -1472,7 +1480,7 @@ struct Engine::Impl {
         int m = TF_CUFFT;
         if (tfWant == TF_AUTO && nsys == 1 && gridOk && fftgKc > 0) {
             const char* dual = std::getenv("PGM_B200_DUAL");
-            if (pcgOk && pcgSmem <= PCG_RULE_SMEM && pmeWant == 0 && !(dual && dual[0] == '1'))
+            if (pcgOk && pcgShared && pcgSmem <= PCG_RULE_SMEM && pmeWant == 0 && !(dual && dual[0] == '1'))
                 m = TF_PCG;
             else if (mixed() || fftgKc < 64 || n <= 12000)
                 m = TF_GRID;
@@ -1485,6 +1493,8 @@ struct Engine::Impl {
             m = TF_GRID;
         if (tfWant == TF_PCG && pcgOk)
             m = TF_PCG;
+        if (m == TF_PCG && !pcgShared)
+            dPcgState.ensure(pcgBlocks * pcgStateBytes((n + pcgBlocks - 1) / pcgBlocks));
         if (m != tfMode && exec) {
             cudaGraphExecDestroy(exec);
             exec = nullptr;

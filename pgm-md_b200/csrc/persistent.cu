@@ -6,7 +6,9 @@
 
 namespace pgmb200 {
 
-PcgKernel pcgKernel(int kc) {
+PcgKernel pcgKernel(int kc, bool shared) {
+    if (!shared)
+        return k_cg_persistent<6, 0, false>;
     switch (kc) {
     case 8: return k_cg_persistent<6, 8>;
     case 9: return k_cg_persistent<6, 9>;

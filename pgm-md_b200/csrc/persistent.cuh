@@ -59,9 +59,13 @@ template <int P> struct PmeRec {
     float c[6 * P];
 };
 
-// Shared memory of a block of `per` slots beside the transforms' tables and buffers (fftgBuf complex elements each).
-__host__ __device__ inline size_t pcgSmemBytes(int per, int fftgBuf) {
-    return (3 * (size_t) FFT_MAXK + 2 * (size_t) fftgBuf) * sizeof(float2) + (size_t) per * (13 * 8 + PCG_SPL * 4 + 4 * 4);
+// Shared memory of a block for the transforms' tables and buffers (fftgBuf complex elements each), and the state of its
+// `per` slots (a multiple of 16 bytes).
+__host__ __device__ inline size_t pcgTransformBytes(int fftgBuf) {
+    return (3 * (size_t) FFT_MAXK + 2 * (size_t) fftgBuf) * sizeof(float2);
+}
+__host__ __device__ inline size_t pcgStateBytes(int per) {
+    return ((size_t) per * (13 * 8 + PCG_SPL * 4 + 4 * 4) + 15) / 16 * 16;
 }
 
 // A load that leaves no line behind in L1 (the pair records, read once per pass).
@@ -164,10 +168,11 @@ __device__ __forceinline__ void pcgTotals(const double* part, int nb, unsigned m
 // KC > 0: the grid is KC^3 (compile-time line transforms); 0: any grid the plane blocks handle.  The right-hand side is
 // E_perm = E_pair + E_rec + self field of the permanent dipoles (written to b), or, with the control's customRhs, b.
 // planeSlots: the rows of the pair pass that a plane block's transforms are worth.
+// SHARED: the slots' state in shared memory; else, for more atoms than that holds, in the block's part of dv.pcgState.
 // finish: also the final pass's preparation (k_final_prep: mu = x + peek alpha r, the total dipoles, the self and
 // polarization energies, the history) and its spread of (q, d), from the state that the blocks hold: two launches
 // and their loads less (480 -> 468 us an evaluation at 4104 atoms, 412 -> 395 at 1900; even at 8550).
-template <int P, int KC>
+template <int P, int KC, bool SHARED = true>
 __global__ void __launch_bounds__(PCG_THREADS, 1) k_cg_persistent(Dev dv, int planeSlots, int finish) {
     typedef cufftComplex C;
     constexpr int SL = PCG_SLOT_LANES;
@@ -186,7 +191,8 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_cg_persistent(Dev dv, int pl
     C* W2 = W1 + FFT_MAXK;
     C* const b0 = W2 + FFT_MAXK;
     C* const b1 = b0 + dv.fftgBuf;
-    double* const sx = (double*) (b1 + dv.fftgBuf);   // the slots' x, r, p, A p (3 per slot), alpha
+    double* const sx = SHARED ? (double*) (b1 + dv.fftgBuf)   // the slots' x, r, p, A p (3 per slot), alpha
+                              : (double*) (dv.pcgState + (size_t) x * pcgStateBytes(per));
     double* const sr = sx + 3 * per;
     double* const sp = sr + 3 * per;
     double* const sAp = sp + 3 * per;

@@ -12,8 +12,9 @@ constexpr int FFTG_MIN_K = 8;
 typedef void (*GridKernel)(Dev, int);
 template <typename R> GridKernel gridKernel(int kc, bool energy);
 
-// The persistent CG kernel, compiled for the cubic grids of pcgSizes; any other grid (kc = 0) takes the general one.
+// The persistent CG kernel, compiled for the same cubic grids; any other grid (kc = 0) takes the general one, and so does an
+// engine of more atoms than the blocks' shared memory holds the state of (shared false: the state in global memory).
 typedef void (*PcgKernel)(Dev, int, int);
-PcgKernel pcgKernel(int kc);
+PcgKernel pcgKernel(int kc, bool shared);
 
 }  // namespace pgmb200

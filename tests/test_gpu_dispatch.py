@@ -46,6 +46,28 @@ def test_persistent_kernel_slot_split(molecules, zero_guess):
         assert np.linalg.norm(a[k] - b[k]) <= 3e-6 * np.linalg.norm(a[k]), k
 
 
+def test_persistent_kernel_beyond_shared_memory():
+    """105000 atoms, whose state the blocks' shared memory does not hold: the rule takes the grid kernel, and a choice of the
+    persistent kernel still runs it, with the results of the graph loop (as above; the zero guess and the solve's)."""
+    S = water(35000, K=64)
+    S.tol = 1e-6
+    out = []
+    for mode in (3, 4):
+        e = engine(S, tol=1e-6)
+        assert e.transforms() == 3
+        e.set_transforms(mode)
+        assert e.transforms() == mode
+        r = e.compute(S.pos, S.box)
+        x, _ = e.solve(e.induced_dipoles(), tol=1e-6)
+        out.append((r.energy, r.iterations, r.forces, r.strain, x))
+        e.close()
+    a, b = out
+    assert abs(a[1] - b[1]) <= 1
+    assert abs(a[0] - b[0]) <= 3e-6 * abs(a[0])
+    for k in (2, 3, 4):
+        assert np.linalg.norm(a[k] - b[k]) <= 3e-6 * np.linalg.norm(a[k]), k
+
+
 def test_persistent_kernel_predicted_steps():
     """Steps of a moving system, each guess of the predictor in turn (none, the last solution, mu3, mu4), with a kept list."""
     S = water(120)
