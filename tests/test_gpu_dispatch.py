@@ -1,6 +1,8 @@
 """The transforms that an engine takes until the caller chooses, and the persistent kernel at the edges of its slot split (fewer
 atoms than blocks, one slot a block, a remainder) and from each initial guess."""
 
+import threading
+
 import numpy as np
 import pytest
 
@@ -143,3 +145,71 @@ def test_other_covalent_dipoles_after_an_evaluation(precision):
         f = fresh.compute(S.pos, S.box)
         assert abs(r.energy - f.energy) <= 1e-12 * abs(f.energy)
         assert np.linalg.norm(r.forces - f.forces) <= 1e-12 * np.linalg.norm(f.forces)
+
+
+GRIDS = [(6, 6, 6), (24, 30, 36), (25, 60, 54), (64, 15, 20), (10, 27, 6), (8, 64, 64), (15, 9, 25)]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("grid", GRIDS, ids=lambda g: "x".join(map(str, g)))
+def test_general_instances_against_cufft(grid, precision):
+    """Whole evaluations by the instances for any grid (three different extents, odd ones, few planes of many lines and many
+    of few): the grid kernel with its energy variant and the persistent kernel against cuFFT's chain, and the solve of another
+    right-hand side.  Mixed: the rounding of float sums in another order, as above; FP64: 64 eps x 18 levels (1.3e-13) of the
+    transforms, carried through some ten iterations and the strain's cancelling terms (100 times that)."""
+    S = PKG.systems.waters(20, 9.0, seed=11, grid=grid, cutoff=4.4, tol=1e-8)
+    lim = 1.3e-11 if precision == 0 else 3e-6
+    out = []
+    for mode in (0, 3, 4) if precision == 1 else (0, 3):
+        e = engine(S, precision=precision)
+        e.set_transforms(mode)
+        assert e.transforms() == mode
+        r = e.compute(S.pos, S.box)
+        mu = e.induced_dipoles()
+        x, _ = e.solve(np.roll(mu, 1, axis=0), tol=1e-8)
+        out.append((r.energy, r.iterations, r.forces, r.strain, mu, x))
+        e.close()
+    for b in out[1:]:
+        a = out[0]
+        assert abs(a[1] - b[1]) <= 1
+        assert abs(a[0] - b[0]) <= lim * abs(a[0])
+        for k in (2, 3, 4, 5):
+            assert np.linalg.norm(a[k] - b[k]) <= lim * np.linalg.norm(a[k]), k
+
+
+def test_engines_in_two_threads():
+    """Engines in threads of their own, each with its cooperative kernels (the persistent one in a compiled and the general
+    instance, the FP64 grid kernel): every evaluation is what the engine computes alone."""
+    cases = [(water(300), 1, None), (water(120), 0, None),
+             (PKG.systems.waters(40, 10.7, seed=4, grid=(24, 30, 36), cutoff=5.0, tol=1e-8), 1, 4)]
+    engines, alone = [], []
+    for S, precision, mode in cases:
+        e = engine(S, precision=precision)
+        if mode is not None:
+            e.set_transforms(mode)
+        engines.append(e)
+        alone.append(e.compute(S.pos, S.box))
+    assert [e.transforms() for e in engines] == [4, 3, 4]
+    wrong = []
+
+    def work(k):
+        S, precision, _ = cases[k]
+        lim = 1e-11 if precision == 0 else 1e-6
+        try:
+            for _ in range(60):
+                r = engines[k].compute(S.pos, S.box)
+                if not (abs(r.energy - alone[k].energy) <= lim * abs(alone[k].energy) and
+                        np.linalg.norm(r.forces - alone[k].forces) <= lim * np.linalg.norm(alone[k].forces)):
+                    wrong.append((k, r.energy, alone[k].energy))
+        except Exception as ex:   # (a thread's error is the test's)
+            wrong.append((k, repr(ex)))
+
+    for pair in ((0, 1), (0, 2), (0, 1, 2)):
+        threads = [threading.Thread(target=work, args=(k,)) for k in pair]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not wrong, (pair, wrong[:3])
+    for e in engines:
+        e.close()
