@@ -230,8 +230,8 @@ int pgm_engine_pair_lanes(pgm_engine* e);
  * barriers (grids as for 1, every system's blocks resident together); 4 that kernel for the passes around the CG solve
  * and the whole solve as one persistent cooperative kernel (mixed precision, one system, order 6).  Until this call one
  * system on a cubic grid of 8 to 64 points with prime factors 2, 3, 5 takes 4 where it applies (up to 85000 to 100000 atoms
- * by grid), else 3 (in FP64 at 64 points up to 12000 atoms), any other grid and batches 0.  The call's choice stands for the
- * engine's life.
+ * by grid), else 3 (in FP64 with 16 or 32 pair lanes, at 64 points up to 12000 atoms), any other grid and batches 0.  The
+ * call's choice stands for the engine's life.
  * pgm_engine_transforms: the kind in use (1 to 4 only where the grids allow them). */
 int pgm_engine_set_transforms(pgm_engine* e, int mode);
 int pgm_engine_transforms(pgm_engine* e);

@@ -1475,6 +1475,8 @@ struct Engine::Impl {
     //     193 KB) 3185 / 3544 / 3621, 98304 (203 KB) 3743 / 3670 / 3779
     //   FP64: 4113 (36^3) - / 493 / 547, 8550 (48^3) - / 935 / 1021, 39000 (60^3) - / 2362 / 2398; 64^3, whose passes take two
     //     rounds of the block's 256 threads: 9000 atoms - / 802 / 850, 15900 - / 1229 / 1210, 26244 - / 1757 / 1711
+    //   FP64 by the pair passes' lanes (32 are the default; with few a long pair pass keeps the grid kernel's blocks waiting),
+    //     8550 atoms (48^3), grid kernel / cuFFT: 32 lanes 937 / 1073, 16 962 / 987, 8 1077 / 1037, 4 1333 / 1208
     // Batches keep cuFFT, whose plans take all systems of a shape at once.
     void selectTransforms() {
         int m = TF_CUFFT;
@@ -1482,7 +1484,7 @@ struct Engine::Impl {
             const char* dual = std::getenv("PGM_B200_DUAL");
             if (pcgOk && pcgShared && pcgSmem <= PCG_RULE_SMEM && pmeWant == 0 && !(dual && dual[0] == '1'))
                 m = TF_PCG;
-            else if (mixed() || fftgKc < 64 || n <= 12000)
+            else if (mixed() || (pairGS >= 16 && (fftgKc < 64 || n <= 12000)))
                 m = TF_GRID;
         }
         if (tfWant == TF_CLUSTER && clusterOk)
@@ -3258,6 +3260,7 @@ void Engine::setPairLanes(int lanes) {
         impl->exec = nullptr;
     }
     impl->pairGS = lanes;
+    impl->selectTransforms();   // (the rule without a caller's choice depends on them in FP64)
 }
 
 int Engine::pairLanes() const { return impl->pairGS; }

@@ -400,8 +400,8 @@ class Engine:
         block per x-plane, 4 that kernel for the field passes around the CG loop and the whole CG loop as one
         persistent cooperative kernel (mixed precision, one system, order 6); transforms() tells which runs.  Until
         this call one system on a cubic grid (8 to 64 points, prime factors 2, 3, 5) takes 4 where it applies (up to 85000
-        to 100000 atoms by grid), else 3 (in FP64 at 64 points up to 12000 atoms), any other grid and a batch 0; the
-        choice stands for the engine's life."""
+        to 100000 atoms by grid), else 3 (in FP64 with 16 or 32 pair lanes, at 64 points up to 12000 atoms), any other grid
+        and a batch 0; the choice stands for the engine's life."""
         _check(self._L.pgm_engine_set_transforms(self._h, int(mode)))
 
     def transforms(self):

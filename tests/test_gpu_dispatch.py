@@ -118,6 +118,20 @@ def test_grids_without_an_instance_keep_cufft(grid, precision):
     e.close()
 
 
+def test_pair_lanes_of_the_rule():
+    """FP64 with few lanes in the pair passes keeps cuFFT until the caller chooses; mixed does not depend on them."""
+    S = water(64, K=16)
+    for precision, modes in ((0, (0, 0, 3, 3)), (1, (4, 4, 4, 4))):
+        e = engine(S, precision=precision)
+        for lanes, mode in zip((4, 8, 16, 32), modes):
+            e.set_pair_lanes(lanes)
+            assert e.transforms() == mode
+        e.set_transforms(3)
+        e.set_pair_lanes(8)
+        assert e.transforms() == 3   # (a choice stands)
+        e.close()
+
+
 @pytest.mark.parametrize("atoms,K,precision,mode", [(85500, 64, 1, 4), (87000, 64, 1, 3), (93000, 48, 1, 4), (98304, 48, 1, 3),
                                                     (12000, 64, 0, 3), (12300, 64, 0, 0), (39000, 60, 0, 3)])
 def test_atom_counts_of_the_rule(atoms, K, precision, mode):
