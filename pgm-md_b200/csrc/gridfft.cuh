@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(FftgThreads<R>::n, FftgThreads<R>::perSm) k_ff
     if (x >= K0)
         return;   // (a smaller grid than the launch's largest)
     const int nT = blockDim.x, tid = threadIdx.x;
+    const int gaveUp = tid == 0 ? dv.flags[11] : 0;   // (its load beside the tables')
     extern __shared__ __align__(16) unsigned char smraw[];
     C* W0 = (C*) smraw;
     C* W1 = W0 + FFT_MAXK;
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(FftgThreads<R>::n, FftgThreads<R>::perSm) k_ff
         W2[m] = tw[S.twOff[2] + m];
     // A barrier of an earlier launch of this call gave up: its counter is out of step, so every wait here would run out too,
     // a second each in every iteration still enqueued.  The results are undefined already; the host reports the flag.
-    if (__syncthreads_or(tid == 0 && dv.flags[11] != 0))
+    if (__syncthreads_or(gaveUp))
         return;
     const PlaneFft<R, KC> fft(K0, K1, K2, b0, b1, W0, W1, W2);
     const int nline = fft.nline, l0 = x * fft.lpb, nl = min(nline, l0 + fft.lpb) - l0;
