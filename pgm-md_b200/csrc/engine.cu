@@ -1473,8 +1473,9 @@ struct Engine::Impl {
     //     general instances' run-time radices, cuFFT stays
     //   PCG_RULE_SMEM, mixed: 85500 atoms (64^3, 193 KB) 3062 / 3199 / 3321, 87000 (196 KB) 3453 / 3259 / 3363; 93000 (48^3,
     //     193 KB) 3185 / 3544 / 3621, 98304 (203 KB) 3743 / 3670 / 3779
-    //   FP64: 4113 (36^3) - / 493 / 547, 8550 (48^3) - / 935 / 1021, 39000 (60^3) - / 2362 / 2398; 64^3, whose passes take two
-    //     rounds of the block's 256 threads: 9000 atoms - / 802 / 850, 15900 - / 1229 / 1210, 26244 - / 1757 / 1711
+    //   FP64: 4113 (36^3) - / 493 / 547, 8550 (48^3) - / 935 / 1021, 39000 (60^3) - / 2362 / 2398; 64^3: 9000 atoms - / 802 /
+    //     850, 15900 - / 1229 / 1210, 26244 - / 1757 / 1711 (alone the transforms take 18.5 us there, cuFFT's 36.4; beside a
+    //     long pair pass the 64 blocks of 72 KB come in late, those of 60^3 with 64 KB do not)
     //   FP64 by the pair passes' lanes (32 are the default; with few a long pair pass keeps the grid kernel's blocks waiting),
     //     8550 atoms (48^3), grid kernel / cuFFT: 32 lanes 937 / 1073, 16 962 / 987, 8 1077 / 1037, 4 1333 / 1208
     // Batches keep cuFFT, whose plans take all systems of a shape at once.

@@ -17,8 +17,9 @@ namespace pgmb200 {
 // The exchange goes through L2, so a 48^3 grid spreads over 48 SMs; loads of what other blocks wrote bypass L1
 // (__ldcg).  Each barrier waits at most FFTG_SPIN_LIMIT polls; a block that gives up sets flags[11] and returns, and
 // the host reports the evaluation as failed.
-// Threads per block: a pass has at most 31 x 10 items (K = 60) or 33 x 8 (K = 64), so 320 threads take any pass of a
-// float grid in one round; 256 in double, so that three blocks fit an SM as many-system launches need them.
+// Threads per block: a pass of a cubic grid has at most 31 x 10 items (K = 60) or 33 x 8 (K = 64), so 320 threads take any of
+// them in one round; 256 in double, so that three blocks fit an SM as many-system launches need them (two rounds at 60 and
+// 64).  Other grids can have more, in more rounds: few planes of many lines take their x-lines so (8 x 64 x 64: 264 lines x 4).
 template <typename R> struct FftgThreads { static constexpr int n = 256, perSm = 3; };
 template <> struct FftgThreads<float> { static constexpr int n = 320, perSm = 2; };
 constexpr unsigned FFTG_SPIN_LIMIT = 1u << 22;   // polls of an L2 word (a few hundred ns each): about 1 s

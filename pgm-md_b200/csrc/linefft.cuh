@@ -189,8 +189,8 @@ template <typename R, int DIR> struct Dft<R, 9, DIR> {
 // exact quotient.
 __device__ __forceinline__ int fdiv(int e, float invK) { return __float2int_rz(((float) e + 0.5f) * invK); }
 
-// The length K of one dimension and its split, compile-time (KC > 0, K = KC) or not, with the division by B or A of
-// a pass's thread index.
+// The length K of one dimension and its split into the two passes' radices, compile-time (KC > 0, K = KC) or not; first and
+// second call f with a pass's radix as a constant (a switch where it is a run-time one).
 template <int KC> struct Split {
     static constexpr int K = KC, A = fftSplitA(KC), B = KC / (fftSplitA(KC) > 0 ? fftSplitA(KC) : 1);
     __device__ __forceinline__ explicit Split(int) {}

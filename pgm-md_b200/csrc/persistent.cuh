@@ -12,7 +12,8 @@
 //   F  blocks 0 .. K0-1 own the x-planes of the PME grid: the plane is read from the fixed-point grid (and cleared for
 //      the next spread), transformed, its share of the x-lines multiplied by the influence function (two barriers of
 //      the plane blocks; linefft.cuh) and transformed back into the potential grid.  The others run the
-//      direct-space field pass of the direction over the pair records (the plane blocks join in when there are many).                                grid barrier
+//      direct-space field pass of the direction over the pair records (the plane blocks join in when there are many).
+//      grid barrier
 //   G  (every block, 16 lanes per slot) E_rec at the atom from the potential grid, the atom's row of A p and the block's
 //      shares of p . A p, z . A p and A p . alpha A p;                                                grid barrier
 //   U  (every block, its own slots) alph = rz / p.Ap, r' = r - alph A p, z' = alpha r'.  The next direction's beta
@@ -47,7 +48,10 @@ constexpr int PCG_SLOT_LANES = 16;           // lanes per slot in the spread and
 // 228 KB and the gathers of the pair pass miss (an evaluation of 85500 atoms at 64^3 takes 3062 us, of 87000 3453).
 constexpr size_t PCG_RULE_SMEM = 198000;
 // Directed pairs that a block sums while a plane block transforms its plane (9.9 us at 48^3): the plane blocks take
-// that many fewer of the pair pass's rows, if any.
+// that many fewer of the pair pass's rows, if any.  Measured at 48^3 and used for every grid; what a third / three times as
+// many would give, us an evaluation: 648 atoms (20^3) 271 / 271 for 271, 12288 (50^3) 679 / 667 for 668, 26244 (64^3) 1073 /
+// 1146 for 1073, 60000 (64^3) 2154 / 2243 for 2173; coarse grids of many atoms would take the lower one, 12288 (32^3) 618 /
+// 631 for 630, 26244 (32^3) 1111 / 1147 for 1127.
 constexpr int PCG_PLANE_PAIRS = 32000;
 constexpr int PCG_SPL = 40;                  // floats per slot of the spline rows: theta, dtheta [3][6], padded so that
                                              // the four slots of a warp read different banks

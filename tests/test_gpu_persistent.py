@@ -1,9 +1,10 @@
-"""The persistent CG kernel (transforms mode 4: the whole mixed-precision CG loop of one system as one
-cooperative launch, PME planes spread, transformed and gathered in shared memory, the direct-space pass on the
-other SMs) against the reference pgm_core's outputs and against the engine's own graph loop (mode 3), on the
-committed goldens: the 216-water box (20^3 grid), the triclinic test box (48^3) and the real 8550-atom
-dimethylphenol liquid (48^3).  Bars as for every mixed path: energy 1e-6, forces 1e-5 relative RMS at tol 1e-10
-against the oracle; the CG iteration count of the graph loop within one."""
+"""The persistent CG kernel (transforms mode 4: the whole mixed-precision solve of one system as one cooperative
+launch with the atoms' vectors in shared memory: the spread into the fixed-point grid, the PME planes' transforms on
+K0 blocks beside the direct-space pass on the others, the gather and the update, and the final pass's preparation)
+against the reference pgm_core's outputs and against the engine's own graph loop (mode 3), on the committed goldens:
+the 216-water box (20^3 grid), the triclinic test box (48^3) and the real 8550-atom dimethylphenol liquid (48^3).
+Bars as for every mixed path: energy 1e-6, forces 1e-5 relative RMS at tol 1e-10 against the oracle; the CG iteration
+count of the graph loop within one."""
 
 import numpy as np
 import pytest
@@ -56,8 +57,8 @@ def test_persistent_cg_against_reference(name, lanes):
 
 
 def test_persistent_cg_repeated_calls_and_tolerance():
-    """The benchmark's tolerance (1e-5) on the 8550-atom liquid, three calls in a row: the same iterations and
-    energies within the mixed path's run-to-run spread (the field passes around the loop use float atomics)."""
+    """The benchmark's tolerance (1e-5) on the 8550-atom liquid, three calls in a row: the same iterations, and
+    energies and forces within the mixed path's bars of the reference each time."""
     S, d = golden("dmp8550_real")
     eng = mixed_engine(S, 4, tol=1e-5)
     rs = [eng.compute(S.pos, S.box) for _ in range(3)]
