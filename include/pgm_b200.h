@@ -158,8 +158,8 @@ int pgm_engine_strain(pgm_engine* e, double* strain);
 int pgm_engine_field(pgm_engine* e, const double* pos, const double* box, const double* q, const double* d,
                      double* E);
 /* The directed pair list of the last evaluation (both directions, r < cutoff by the reference's minimum
- * image, core/pgm_core.cpp:64-87): pairs i < j written to pi, pj (capacity cap); *npairs = count.  No
- * counterpart in the reference (its list is internal). */
+ * image, core/pgm_core.cpp:64-87): pairs i < j written to pi, pj (capacity cap); *npairs = count
+ * (0 before an evaluation).  No counterpart in the reference (its list is internal). */
 int pgm_engine_pairs(pgm_engine* e, int* pi, int* pj, long long cap, long long* npairs);
 
 /* Predictor history as a blob (checkpoint/resume): size in bytes, get, set.  No counterpart in the

@@ -243,6 +243,7 @@ struct Engine::Impl {
     // Verlet list state: valid once built; kept while the boxes stay those of the build and no atom has moved by
     // more than half the skin (checked on the device at every evaluation)
     bool listValid = false;
+    bool rowsValid = false;      // the list's rows hold the pairs of an evaluation (not since set-up or a growth)
     bool externalList = false;   // the caller's candidates (setCandidates) in place of the cell search
     // the combination-rule GVDW (setGvdw)
     bool gvdwOn = false, gvdwSlater = false;
@@ -879,6 +880,7 @@ struct Engine::Impl {
         uploadCovalent();
         haveResult = false;
         listValid = false;
+        rowsValid = false;
         configured = true;
     }
 
@@ -968,6 +970,7 @@ struct Engine::Impl {
 
     void allocList() {
         listValid = false;
+        rowsValid = false;
         dList.ensure((size_t) n * cap * sizeof(uint32_t));
         dSList.ensure((size_t) n * cap * sizeof(uint32_t));
         if (mixed())   // pair records: (x, G1) + (G2, slot of j) in float; FP64 (G1, G2) only
@@ -2234,6 +2237,7 @@ struct Engine::Impl {
         }
         lastResults.assign(hResults, hResults + nsys * NRES);
         haveResult = true;
+        rowsValid = true;
         if (nsys == 1 && s.polarizable) {   // the unroll of the next capture
             recentIt[recentCount++ % 4] = (int) hResults[14];
             evalsSinceCapture++;
@@ -2621,6 +2625,8 @@ void Engine::resetHistory() { impl->resetHistoryState(); }
 long Engine::listBuilds() const { return impl->builds; }
 
 int Engine::numCandidates() const {
+    if (!impl->rowsValid)
+        return 0;
     std::vector<int> c(impl->n);
     CU(cudaMemcpy(c.data(), impl->dListCount.p, impl->n * sizeof(int), cudaMemcpyDeviceToHost));
     long long s = 0;
@@ -2639,6 +2645,8 @@ std::array<double, 9> Engine::strainDerivative() const {
 
 long long Engine::pairs(int* pi, int* pj, long long cap) {
     Impl& I = *impl;
+    if (!I.rowsValid)
+        return 0;
     std::vector<int> cnt(I.n), slotAtom(I.n);
     std::vector<uint32_t> list((size_t) I.n * I.cap);
     CU(cudaMemcpy(cnt.data(), I.dListCount.p, I.n * sizeof(int), cudaMemcpyDeviceToHost));
@@ -2746,6 +2754,7 @@ void Engine::field(const double* pos, const double box[3][3], const double* qf, 
         for (size_t k = 0; k < 3 * (size_t) I.n; k++)
             E[k] = ep[k] + er[k] + cs * d[k];
         I.haveResult = false;
+        I.rowsValid = true;
         return;
     }
     throw std::runtime_error("pgm_b200: pair list did not fit after growing it");
@@ -2879,6 +2888,7 @@ Terms Engine::evaluateFixed(const double* pos, const double box[3][3], const dou
         }
         I.lastResults.assign(I.hResults, I.hResults + I.nsys * NRES);
         I.haveResult = true;
+        I.rowsValid = true;
         I.hCtl->fixedMu = 0;
         return I.termsOf(0);
     }

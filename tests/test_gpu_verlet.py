@@ -86,3 +86,19 @@ def test_skin_zero_builds_every_evaluation():
         assert rel_rms(a.forces, b.forces) <= 1e-12
     assert kept.list_builds() == 1
     assert fresh.list_builds() == 3
+
+
+@pytest.mark.parametrize("precision", [PKG.FP64, PKG.MIXED])
+def test_pairs_before_an_evaluation(precision):
+    """No evaluation, no pairs: after set-up and after new atoms (the rows then hold whatever the memory held)."""
+    S = water512()
+    e = make_engine(S, precision)
+    assert e.num_candidates() == 0 and len(e.pairs()[0]) == 0
+    e.compute(S.pos, S.box)
+    found = len(e.pairs()[0])
+    assert found > 0 and e.num_candidates() == 2 * found
+    e.set_system(S)
+    assert e.num_candidates() == 0 and len(e.pairs()[0]) == 0
+    e.field(S.pos, S.box, S.q, np.zeros((S.n, 3)))
+    assert len(e.pairs()[0]) == found
+    e.close()
