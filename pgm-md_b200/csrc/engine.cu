@@ -3112,18 +3112,22 @@ int Engine::kernelLaunches() const {
     const Impl& I = *impl;
     if (!I.haveResult)
         return 0;
-    // own kernels per evaluation (the cuFFT transforms not counted): with a kept list preparation 7 and the Verlet
+    // own kernels per evaluation (the cuFFT transforms and the plane tiles' further kernels not counted): with a kept list preparation 7 and the Verlet
     // list's build 5 when it ran, without a skin 9; a field pass fp = 4 (spread, the transform kernel or the influence
-    // product, pair pass, gather); polarizable: two field passes + 2 before the loop, fp + 2 per CG iteration (fp + 1 with
-    // A p in the gather), or one pass and one launch for the whole solve; final 6
+    // product, pair pass, gather) and the fixed-point grid's conversion where the transforms do not read it; polarizable: two
+    // field passes + 2 before the loop (without a skin the first one's pair pass is the records'), fp + 2 per CG iteration
+    // (fp + 1 with A p in the gather), or one pass and one launch for the whole solve (not with the refinement, which runs
+    // the loop's kernels); final 6 and the conversion, or 4 after the whole solve
     int it = 0;
     for (int k = 0; k < I.nsys; k++)
         it = std::max(it, (int) I.lastResults[(size_t) k * NRES + 14]);
-    const int fp = 4, perIt = fp + (I.fusedGather() ? 1 : 2);
+    const int conversion = I.spreadFix() && I.tfMode != Impl::TF_GRID && I.tfMode != Impl::TF_PCG ? 1 : 0;
+    const int fp = 4 + conversion, perIt = fp + (I.fusedGather() ? 1 : 2);
     const int pre = I.verletList() ? 7 + (I.lastBuilt ? 5 : 0) : 9;
-    const bool pcg = I.s.polarizable && I.persistentMode();
-    const int solve = !I.s.polarizable ? 0 : pcg ? fp + 1 : 2 * fp + 2 + perIt * it;
-    return pre + solve + (pcg && I.spreadFix() ? 4 : 6) + (I.gvdwOn ? 1 : 0);
+    const bool pcg = I.s.polarizable && I.persistentMode() && !I.refining();
+    const int first = fp - (I.verletList() || I.dualFirstPass() ? 0 : 1);
+    const int solve = !I.s.polarizable ? 0 : pcg ? first + 1 : first + fp + 2 + perIt * it;
+    return pre + solve + (pcg && I.spreadFix() ? 4 : 6 + conversion) + (I.gvdwOn ? 1 : 0);
 }
 
 void Engine::kernelTimes(int reps, double* ms, void* flush, size_t flushBytes) {

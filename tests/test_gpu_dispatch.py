@@ -227,3 +227,17 @@ def test_engines_in_two_threads():
         assert not wrong, (pair, wrong[:3])
     for e in engines:
         e.close()
+
+
+def test_kernel_launches_counted():
+    """The launch count of each solve: without a skin 9 to the records, the permanent field 3, the persistent kernel 1 and the
+    final pass 4; the graph loop 3 + 4 + 2, 5 an iteration and 6; with cuFFT the fixed-point grid's conversion in each pass.
+    With the refinement the loop's kernels run whatever the mode."""
+    S = water(64, K=16)
+    for mode, refine, count in ((4, False, lambda it: 17), (3, False, lambda it: 24 + 5 * it), (0, False, lambda it: 27 + 6 * it),
+                                (4, True, lambda it: 24 + 5 * it), (3, True, lambda it: 24 + 5 * it)):
+        e = engine(S, tol=1e-6, skin=0.0, refine=refine)
+        e.set_transforms(mode)
+        r = e.compute(S.pos, S.box)
+        assert e.kernel_launches() == count(r.iterations), (mode, refine)
+        e.close()
